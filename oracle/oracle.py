@@ -30,7 +30,7 @@ def build(ref: bool = True) -> None:
     """Build the oracle library (always) and the reference binaries (when the
     reference sources are present)."""
     subprocess.run(["make", "-C", str(HERE), "-s"], check=True)
-    if ref and REFERENCE_SRC.exists():
+    if ref and (REFERENCE_SRC / "main.cpp").exists():  # an empty folder holds no sources
         subprocess.run(["make", "-C", str(HERE), "-s", "-j8", "ref", f"REF={REFERENCE_SRC}"], check=True)
 
 
