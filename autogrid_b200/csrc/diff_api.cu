@@ -114,14 +114,11 @@ struct ag_diff {
 
 namespace {
 
-// vdW rows [type][bin][stride]: slot s holds the table of its atom map
-// (slot_tab[s]; zero for slots without a pair term).
-template <class R>
-void build_tables(const ag_problem *p, const DiffArgs &A, std::vector<R2<R>> &vdw, std::vector<R2<R>> &sol,
-                  std::vector<R2<R>> &eps)
+// Every vdW table entry: put(type * NEINT + bin, slot, value, step to the next
+// bin); slot s takes the table of its atom map (slot_tab[s]).
+template <class Put> void each_vdw(const ag_problem *p, const DiffArgs &A, Put put)
 {
-    const int nT = p->n_rec_types, nAM = p->n_atom_maps, W = A.tab_stride;
-    vdw.assign((size_t)std::max(nT, 1) * AG_NEINT * W, R2<R>{R(0), R(0)});
+    const int nT = p->n_rec_types, nAM = p->n_atom_maps;
     for (int t = 0; t < nT; t++)
         for (int s = 0; s < A.n_slots; s++) {
             const int m = A.slot_tab[s];
@@ -129,9 +126,14 @@ void build_tables(const ag_problem *p, const DiffArgs &A, std::vector<R2<R>> &vd
             const float *src = p->e_vdw_hb + ((size_t)t * nAM + m) * AG_NEINT;
             for (int b = 0; b < AG_NEINT; b++) {
                 const double v = src[b], nx = (b < AG_NEINT - 1) ? (double)src[b + 1] : v;
-                vdw[((size_t)t * AG_NEINT + b) * W + s] = R2<R>{R(v), R(nx - v)};
+                put((size_t)t * AG_NEINT + b, s, v, nx - v);
             }
         }
+}
+
+template <class R>
+void build_tables(const ag_problem *p, std::vector<R2<R>> &sol, std::vector<R2<R>> &eps)
+{
     sol.resize(AG_NEINT);
     for (int b = 0; b < AG_NEINT; b++)
         sol[b] = R2<R>{R(p->sol_fn[b]), R(p->sol_fn[b + 1] - p->sol_fn[b])};
@@ -331,6 +333,9 @@ ag_status ag_diff_create_batch(ag_context *ctx, const ag_problem *p, const ag_op
         slots.push_back(s);
     }
     if (need_h && st == AG_ERR_NO_CLOSEST_H) return st;
+    // slots with H-bond actions first, those with a min/max before the others
+    auto has_hb = [](const Slot &s) { return std::any_of(s.act, s.act + 16, [](uint8_t a) { return act_uses_angles(a); }); };
+    std::stable_partition(slots.begin(), slots.end(), [&](const Slot &s) { return s.mm || has_hb(s); });
     std::stable_partition(slots.begin(), slots.end(), [](const Slot &s) { return s.mm; });
     const int n_mm = (int)std::count_if(slots.begin(), slots.end(), [](const Slot &s) { return s.mm; });
     if ((int)slots.size() > DF_MAXS || n_mm > DF_MAXMM) {
@@ -411,6 +416,16 @@ ag_status ag_diff_create_batch(ag_context *ctx, const ag_problem *p, const ag_op
         std::memcpy(A.act[s], sl.act, 16);
         if (sl.kind == DK_D || sl.desolv) A.need_sol = 1;
     }
+    A.row_stride = (A.n_slots + 7) / 8 * 8;
+    A.n_hb = (int)std::count_if(slots.begin(), slots.end(), has_hb);
+    for (int c = 0; c < 16; c++) {
+        bool plain = true;
+        for (int s = 0; s < A.n_slots; s++) {
+            A.cls_act[c] |= (unsigned long long)A.act[s][c] << (4 * s);
+            plain &= !act_uses_angles(A.act[s][c]);
+        }
+        if (plain) A.cls_plain |= 1u << c;
+    }
     // cell list geometry: at most 6 cells per axis around a brick
     const double span = (DF_BRICK_X - 1) * p->spacing + 2 * DF_RADIUS;
     A.cell_size = std::max(4.0, span / 5.0);
@@ -438,14 +453,23 @@ ag_status ag_diff_create_batch(ag_context *ctx, const ag_problem *p, const ag_op
     DF_CK(cudaMemcpy(d->d_meta, meta.data(), N * sizeof(int), cudaMemcpyHostToDevice));
     if (!d->h_index.empty())
         DF_CK(cudaMemcpy(d->d_h, d->h_index.data(), d->h_index.size() * sizeof(int), cudaMemcpyHostToDevice));
+    const size_t n_rows = (size_t)std::max(p->n_rec_types, 1) * AG_NEINT;
     if (d->fp64) {
-        std::vector<R2<double>> vdw, sol, eps;
-        build_tables(p, A, vdw, sol, eps);
+        std::vector<R2<double>> vdw(n_rows * A.tab_stride, R2<double>{0.0, 0.0}), sol, eps;
+        each_vdw(p, A, [&](size_t row, int s, double v, double dv) { vdw[row * A.tab_stride + s] = R2<double>{v, dv}; });
+        build_tables(p, sol, eps);
         DF_CK(put(&d->d_vdw, vdw, d.get())); DF_CK(put(&d->d_sol, sol, d.get())); DF_CK(put(&d->d_eps, eps, d.get()));
     } else {
-        std::vector<R2<float>> vdw, sol, eps;
-        build_tables(p, A, vdw, sol, eps);
-        DF_CK(put(&d->d_vdw, vdw, d.get())); DF_CK(put(&d->d_sol, sol, d.get())); DF_CK(put(&d->d_eps, eps, d.get()));
+        std::vector<float> rows(2 * n_rows * A.row_stride, 0.f);  // values, then steps
+        each_vdw(p, A, [&](size_t row, int s, double v, double dv) {
+            rows[row * A.row_stride + s] = (float)v;
+            rows[(n_rows + row) * A.row_stride + s] = (float)dv;
+        });
+        std::vector<R2<float>> sol, eps;
+        build_tables(p, sol, eps);
+        DF_CK(put(&d->d_vdw, rows, d.get())); DF_CK(put(&d->d_sol, sol, d.get())); DF_CK(put(&d->d_eps, eps, d.get()));
+        A.row_v = (const float *)d->d_vdw;
+        A.row_d = A.row_v + n_rows * A.row_stride;
     }
     A.x = d->d_x; A.y = d->d_y; A.z = d->d_z; A.q = d->d_q; A.vol = d->d_vol; A.solpar = d->d_solpar;
     A.rv = d->d_rv; A.rv2 = d->d_rv2; A.meta = d->d_meta; A.h_index = d->d_h;
@@ -520,7 +544,8 @@ ag_status ag_diff_forward(ag_diff *d, int32_t keep_closest_h, void *device_out)
     }
     DF_CK(cudaEventRecord(d->ev[0], s));
     if (d->elec >= 0) DF_CK(launch_emap_lin(d->fp64, A, d->d_eps, out + d->esz * d->P * d->elec, s));
-    DF_CK(launch_near_lin(d->fp64, A, d->d_vdw, d->d_sol, out, d->d_ch, d->d_mmarg, s));
+    if (d->fp64) DF_CK(launch_near_lin(A, d->d_vdw, d->d_sol, (double *)out, d->d_ch, d->d_mmarg, s));
+    else DF_CK(launch_rows(A, d->d_sol, (float *)out, d->d_ch, d->d_mmarg, s));
     if (d->floating || d->constriction)
         for (int k = 0; k < d->n_conf; k++) {
             // floating and constriction grids of conformer k (FP64, the reference's distances)
@@ -596,7 +621,10 @@ ag_status ag_diff_backward(ag_diff *d, const void *grad_maps, int32_t grad_on_de
     DF_CK(cudaMemsetAsync(d->d_grad, 0, 10 * N * K * sizeof(double), s));
     DF_CK(cudaEventRecord(d->ev[2], s));
     if (d->elec >= 0) DF_CK(launch_emap_lin_adj(d->fp64, d->args, d->d_eps, gm + d->esz * d->P * d->elec, g, s));
-    DF_CK(launch_near_lin_adj(d->fp64, d->args, d->d_vdw, d->d_sol, gm, d->d_ch, d->d_mmarg, g, s));
+    if (d->fp64)
+        DF_CK(launch_near_lin_adj(d->args, d->d_vdw, d->d_sol, (const double *)gm, d->d_ch, d->d_mmarg, g, s));
+    else
+        DF_CK(launch_rows_adj(d->args, d->d_sol, (const float *)gm, d->d_ch, d->d_mmarg, g, s));
     if (d->floating)  // the constriction grid is piecewise constant: no gradient
         for (size_t k = 0; k < K; k++)
             DF_CK(launch_fmap_adjoint(d->conformer_geometry((int)k),

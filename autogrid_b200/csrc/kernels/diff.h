@@ -29,8 +29,6 @@ namespace agb {
 
 constexpr int DF_MAXS = 16;   // map slots of the short-range kernels (atom maps, desolvation partners, d)
 constexpr int DF_MAXMM = 8;   // slots that keep an H-bond min/max
-constexpr int DF_LEAN_S = 8;  // slots of the lean kernel instantiations
-constexpr int DF_MID_MM = 2;  // min/max registers of the middle one (the lean one has none)
 constexpr int DF_BRICK_X = 8, DF_BRICK_Y = 8, DF_BRICK_Z = 4;
 constexpr int DF_THREADS = DF_BRICK_X * DF_BRICK_Y * DF_BRICK_Z;
 constexpr int DF_STAGE = 256;       // candidate atoms staged in shared memory at once
@@ -84,6 +82,14 @@ struct DiffArgs {
     int slot_desolv[DF_MAXS];    // 1: receives a desolvation term
     double slot_sp[DF_MAXS], slot_vp[DF_MAXS];
     uint8_t act[DF_MAXS][16];    // [slot][hbond + 8 * disorder]
+    // FP32 kernels (diff_rows.cu): value and step rows [type][bin][row_stride],
+    // row_stride a multiple of 8; the actions of a class, 4 bits per slot; the
+    // classes whose every slot is plain; slots [0, n_hb) hold every slot with
+    // an H-bond action
+    const float *row_v, *row_d;
+    int row_stride, n_hb;
+    unsigned cls_plain;
+    unsigned long long cls_act[16];
     double cov_pos[3], cov_half_width, cov_barrier;
     int elec_map;
 };
@@ -93,8 +99,9 @@ constexpr int DM_DIS = 1 << 11, DM_SKIP = 1 << 12;
 
 // Interpolation tables, (value, next - value) per bin, in the working
 // precision: vdw [n_rec_types][NEINT][tab_stride] (slot s of a row holds the
-// table of the slot's atom map, so one pair's slots are one contiguous read),
-// sol [NEINT], eps [NDIEL] (dielectric factor * coeff_estat).
+// table of the slot's atom map, so one pair's slots are one contiguous read;
+// FP64 only, the FP32 kernels read row_v and row_d), sol [NEINT], eps [NDIEL]
+// (dielectric factor * coeff_estat).
 template <class R> struct R2 { R v, d; };
 
 struct DiffGrads {
@@ -135,9 +142,13 @@ cudaError_t launch_cell_lists(const DiffArgs &a, int *cell_of, int *count, cudaS
 cudaError_t launch_emap_lin(bool fp64, const DiffArgs &a, const void *eps, void *emap, cudaStream_t s);
 cudaError_t launch_emap_lin_adj(bool fp64, const DiffArgs &a, const void *eps, const void *g_e, DiffGrads g,
                                 cudaStream_t s);
-cudaError_t launch_near_lin(bool fp64, const DiffArgs &a, const void *vdw, const void *sol, void *maps,
-                            const int *ch, int *mmarg, cudaStream_t s);
-cudaError_t launch_near_lin_adj(bool fp64, const DiffArgs &a, const void *vdw, const void *sol, const void *g_maps,
-                                const int *ch, const int *mmarg, DiffGrads g, cudaStream_t s);
+// The FP64 twin (kernels/diff_near.cu) and the FP32 kernels (kernels/diff_rows.cu).
+cudaError_t launch_near_lin(const DiffArgs &a, const void *vdw, const void *sol, double *maps, const int *ch, int *mmarg,
+                            cudaStream_t s);
+cudaError_t launch_near_lin_adj(const DiffArgs &a, const void *vdw, const void *sol, const double *g_maps, const int *ch,
+                                const int *mmarg, DiffGrads g, cudaStream_t s);
+cudaError_t launch_rows(const DiffArgs &a, const void *sol, float *maps, const int *ch, int *mmarg, cudaStream_t s);
+cudaError_t launch_rows_adj(const DiffArgs &a, const void *sol, const float *g_maps, const int *ch, const int *mmarg,
+                            DiffGrads g, cudaStream_t s);
 
 }  // namespace agb

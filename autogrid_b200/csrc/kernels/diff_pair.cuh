@@ -327,12 +327,11 @@ template <class R> struct Term {
     R v, dT, dTH, dracc, drdon, dH, dx;  // dx: total d v / d x through both tables
 };
 
-// te: the pair's table entry (value, slope) for slot s.
-template <class R>
-DF_HD void term(const DiffArgs &a, const R2<R> *vdw, int act, const R2<R> &te, int s, const Geom<R> &g,
-                const Ang<R> &an, Term<R> &t)
+// T and dT_x: the pair's interpolated table value and its slope per bin;
+// th(slope): T_H and its slope, evaluated for the disordered actions only.
+template <class R, class TH>
+DF_HD void term_of(int act, R T, R dT_x, const Ang<R> &an, TH th, Term<R> &t)
 {
-    const R T = lerp(te, g.fx);
     R drs;
     const R rs = rsph(T, drs);
     t.dT = R(0); t.dTH = R(0); t.dracc = R(0); t.drdon = R(0); t.dH = R(0);
@@ -349,13 +348,13 @@ DF_HD void term(const DiffArgs &a, const R2<R> *vdw, int act, const R2<R> &te, i
             t.dH = T * f;
         } break;
         case DA_SUMA_DIS: {
-            const R TH = th_lookup(a, vdw, s, g.x, dth);
+            const R TH_ = th(dth);
             const R f = an.racc + (R(1) - an.racc) * rs;
-            t.v = TH * an.H * f;
+            t.v = TH_ * an.H * f;
             t.dTH = an.H * f;
-            t.dT = TH * an.H * (R(1) - an.racc) * drs;
-            t.dracc = TH * an.H * (R(1) - rs);
-            t.dH = TH * f;
+            t.dT = TH_ * an.H * (R(1) - an.racc) * drs;
+            t.dracc = TH_ * an.H * (R(1) - rs);
+            t.dH = TH_ * f;
         } break;
         case DA_MMA: {
             const R f = an.racc + (R(1) - an.racc) * rs;
@@ -364,13 +363,13 @@ DF_HD void term(const DiffArgs &a, const R2<R> *vdw, int act, const R2<R> &te, i
             t.dracc = T * (R(1) - rs);
         } break;
         case DA_SUMD_DIS: {
-            const R TH = th_lookup(a, vdw, s, g.x, dth);
+            const R TH_ = th(dth);
             const R f = an.rdon + (R(1) - an.rdon) * rs;
-            t.v = TH * an.H * f;
+            t.v = TH_ * an.H * f;
             t.dTH = an.H * f;
-            t.dT = TH * an.H * (R(1) - an.rdon) * drs;
-            t.drdon = TH * an.H * (R(1) - rs);
-            t.dH = TH * f;
+            t.dT = TH_ * an.H * (R(1) - an.rdon) * drs;
+            t.drdon = TH_ * an.H * (R(1) - rs);
+            t.dH = TH_ * f;
         } break;
         case DA_MMD: {
             const R f = an.rdon + (R(1) - an.rdon) * rs;
@@ -382,30 +381,23 @@ DF_HD void term(const DiffArgs &a, const R2<R> *vdw, int act, const R2<R> &te, i
             t.v = R(0);
             break;
     }
-    t.dx = t.dT * te.d + t.dTH * dth;
+    t.dx = t.dT * dT_x + t.dTH * dth;
+}
+
+// te: the pair's table entry (value, slope) for slot s.
+template <class R>
+DF_HD void term(const DiffArgs &a, const R2<R> *vdw, int act, const R2<R> &te, int s, const Geom<R> &g,
+                const Ang<R> &an, Term<R> &t)
+{
+    term_of(act, lerp(te, g.fx), te.d, an, [&](R &dth) { return th_lookup(a, vdw, s, g.x, dth); }, t);
 }
 
 DF_HD bool act_is_mm(int act) { return act == DA_MMA || act == DA_MMD; }
 
-// The first n (<= MS) entries of a table row.  FP32 on the device reads two
-// slots per 16-byte load: rows hold tab_stride (a multiple of 4) entries of
-// 8 bytes, so every row starts 16-byte aligned.
+// The first n (<= MS) entries of a table row.
 template <class R, int MS>
 DF_HD void load_row(const R2<R> *row, int n, R2<R> *out)
 {
-#ifdef __CUDA_ARCH__
-    if constexpr (sizeof(R) == 4 && MS % 2 == 0) {
-        const float4 *r4 = reinterpret_cast<const float4 *>(row);
-#pragma unroll
-        for (int k = 0; k < MS / 2; k++)
-            if (2 * k < n) {
-                const float4 v = __ldg(r4 + k);
-                out[2 * k] = R2<R>{v.x, v.y};
-                out[2 * k + 1] = R2<R>{v.z, v.w};
-            }
-        return;
-    }
-#endif
 #pragma unroll
     for (int s = 0; s < MS; s++)
         if (s < n) out[s] = row[s];
