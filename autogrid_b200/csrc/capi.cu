@@ -391,6 +391,25 @@ cudaError_t upload(BufferSet *b, const char *name, const T *src, size_t n, T **d
     return e;
 }
 
+// Error bounds of the canonical FP32 distances for a grid spacing (in bins):
+// the far kernel's bin-guard multipliers and the near kernel's guard, from the
+// largest frame-relative point coordinate and whether every frame point
+// coordinate il*spacing_adiv is an exact float.  rsqrt.approx.f32 is taken at
+// 2.5 * 2^-24 relative error (PTX ISA: 2^-22.9 = 2.14 * 2^-24; checked on the
+// device by ag_diag_rsqrt_error).
+void far_guard(double spacing_adiv, float *lo, float *hi, float *near)
+{
+    bool exact = true;
+    for (int il = 0; il < FRAME_X; il++) {
+        const double v = (double)il * spacing_adiv;
+        exact &= std::fma((double)il, spacing_adiv, -v) == 0.0 && (double)(float)v == v;
+    }
+    const double px = (FRAME_X - 1) * spacing_adiv, pyz = (FRAME_Y - 1) * spacing_adiv;
+    const double p_max = std::sqrt(px * px + 2 * pyz * pyz);
+    far_edge_multipliers(p_max, exact, 2.5, lo, hi);
+    *near = near_edge_guard(p_max, exact, 2.5);
+}
+
 // Build the device image of a problem (host work is O(atoms + tables)).
 ag_status launch_far_slab(ag_plan *pl, cudaStream_t s, int k, int nslab);
 
@@ -416,6 +435,10 @@ ag_status build_plan(ag_plan *pl, const ag_problem *p, cudaStream_t s, bool pipe
     for (int i = 0; i < 3; i++) d.cov_pos[i] = p->cov_pos[i];
     d.cov_half_width = p->cov_half_width; d.cov_barrier = p->cov_barrier;
     d.report_collisions = p->report_collisions ? 1 : 0;
+    {
+        float lo, hi;
+        far_guard(d.spacing * AG_A_DIV, &lo, &hi, &d.near_guard);
+    }
     pl->h2d_bytes = 0;
     size_t *acc = &pl->h2d_bytes;
 
@@ -580,7 +603,9 @@ ag_status build_plan(ag_plan *pl, const ag_problem *p, cudaStream_t s, bool pipe
 
     // map groups in kernel order (actions after main.cpp:3286-3379).  Maps that
     // keep an hbond min/max for some receptor class go first, at most NG_MM per
-    // launch, so their min/max accumulators have fixed register slots.
+    // launch, so their min/max accumulators have fixed slots; then the other
+    // maps with an H-bond action, so that these share as few 4-map table rows
+    // as possible (other rows add as a whole, NearGroup::plain4).
     std::vector<int> is_partner(std::max(nAM, 1), 0);
     if (p->separate_desolvation_maps) {
         for (int m = 0; m < nAM; m++) {
@@ -590,10 +615,10 @@ ag_status build_plan(ag_plan *pl, const ag_problem *p, cudaStream_t s, bool pipe
         }
     }
     std::vector<std::array<uint8_t, 8>> act(std::max(nAM, 1));
-    std::vector<int> mm_maps, plain_maps;
+    std::vector<int> mm_maps, sum_maps, plain_maps;
     for (int m = 0; m < nAM; m++) {
         const bool aff = !p->map_is_covalent[m] && !is_partner[m];
-        bool mm = false;
+        bool mm = false, hbond = false;
         for (int hb = 0; hb < 8; hb++) {
             uint8_t a = ACT_PLAIN;
             if (!aff) a = ACT_SKIP;
@@ -605,9 +630,11 @@ ag_status build_plan(ag_plan *pl, const ag_problem *p, cudaStream_t s, bool pipe
             }
             act[m][hb] = a;
             if (hb <= 6 && (a == ACT_MMA || a == ACT_MMD)) mm = true;
+            if (a == ACT_SUMA || a == ACT_MMA || a == ACT_MMD) hbond = true;
         }
-        (mm ? mm_maps : plain_maps).push_back(m);
+        (mm ? mm_maps : hbond ? sum_maps : plain_maps).push_back(m);
     }
+    plain_maps.insert(plain_maps.begin(), sum_maps.begin(), sum_maps.end());
     pl->groups.clear();
     pl->any_cov = false;
     std::vector<uint8_t> skip_map(std::max(nAM, 1), 0);  // ACT_SKIP for every class: table column left zero
@@ -621,7 +648,7 @@ ag_status build_plan(ag_plan *pl, const ag_problem *p, cudaStream_t s, bool pipe
         g.ng = (int)order.size();
         g.write_special = pl->groups.empty() ? 1 : 0;
         g.has_hrow = p->disorder_h ? 1 : 0;
-        g.col0 = (int)pl->groups.size() * NG_MAX;
+        g.col0 = pl->groups.empty() ? 0 : pl->groups.back().col0 + (pl->groups.back().ng + 7) / 8 * 8;
         for (int k = 0; k < g.ng; k++) {
             const int m = order[k];
             g.out_map[k] = m;
@@ -655,7 +682,8 @@ ag_status build_plan(ag_plan *pl, const ag_problem *p, cudaStream_t s, bool pipe
     } while (im < mm_maps.size() || ip < plain_maps.size());
 
     // tables: vdW/H-bond transposed to [type][bin][column], columns in kernel order
-    pl->mpad = (int)pl->groups.size() * NG_MAX;
+    // (whole 32-byte rows of 8 columns)
+    pl->mpad = pl->groups.back().col0 + std::max(8, (pl->groups.back().ng + 7) / 8 * 8);
     const int nT = std::max(1, p->n_rec_types);
     std::vector<int> colmap(pl->mpad, -1);
     for (const NearGroup &g : pl->groups)
@@ -785,22 +813,6 @@ ag_status build_plan(ag_plan *pl, const ag_problem *p, cudaStream_t s, bool pipe
     return AG_OK;
 }
 
-// Bin-guard multipliers of the far kernel for a grid spacing (in bins):
-// far_edge_multipliers with the largest frame-relative point coordinate and
-// whether every frame point coordinate il*spacing_adiv is an exact float.
-// rsqrt.approx.f32 is taken at 2.5 * 2^-24 relative error (PTX ISA:
-// 2^-22.9 = 2.14 * 2^-24; checked on the device by ag_diag_rsqrt_error).
-void far_guard(double spacing_adiv, float *lo, float *hi)
-{
-    bool exact = true;
-    for (int il = 0; il < FRAME_X; il++) {
-        const double v = (double)il * spacing_adiv;
-        exact &= std::fma((double)il, spacing_adiv, -v) == 0.0 && (double)(float)v == v;
-    }
-    const double px = (FRAME_X - 1) * spacing_adiv, pyz = (FRAME_Y - 1) * spacing_adiv;
-    far_edge_multipliers(std::sqrt(px * px + 2 * pyz * pyz), exact, 2.5, lo, hi);
-}
-
 FarArgs far_args(const ag_plan *pl)
 {
     const DevProblem &d = pl->dp;
@@ -817,7 +829,8 @@ FarArgs far_args(const ag_plan *pl)
     a.tab_full = pl->far_tab ? pl->far_tab + pl->tab_len : nullptr;
     a.tab_len = pl->far_mode == FAR_TAB_CONST ? 0 : pl->tab_len;
     a.clamp = pl->far_clamp;
-    far_guard(a.spacing_adiv, &a.edge_lo, &a.edge_hi);
+    float near;
+    far_guard(a.spacing_adiv, &a.edge_lo, &a.edge_hi, &near);
     a.edge_bits = pl->edge_bits;
     a.edge_words = far_edge_words(pl->chunk_atoms);
     a.edge_counters = pl->ctx ? pl->ctx->d_counters + 2 : nullptr;
@@ -884,7 +897,7 @@ ag_status enqueue_slabs(ag_plan *pl, cudaStream_t s, int nslab, int &launches)
         const int bz0 = sz0 / 4, bz1 = (k == nslab - 1) ? -1 : sz1 / 4;  // 8x8x4 bricks
         if (need_near)
             for (const NearGroup &g : pl->groups) {
-                AGB_CK(launch_near(false, d, g, near_ptrs(pl, c->d_counters), 0, s, bz0, bz1));
+                AGB_CK(launch_near(d, g, near_ptrs(pl, c->d_counters), s, bz0, bz1));
                 launches++;
             }
         if (far) {
@@ -970,7 +983,7 @@ ag_status run_plan_zrange(ag_plan *pl, cudaStream_t s, int z0, int z1)
     const bool need_near = d.n_atom_maps > 0 || d.dsolv_map >= 0 || d.elec_map >= 0;
     if (need_near)
         for (const NearGroup &g : pl->groups) {
-            AGB_CK(launch_near(false, d, g, near_ptrs(pl, c->d_counters), 0, s, z0 / 4, last ? -1 : z1 / 4));
+            AGB_CK(launch_near(d, g, near_ptrs(pl, c->d_counters), s, z0 / 4, last ? -1 : z1 / 4));
             launches++;
         }
     if (far) {
@@ -1047,7 +1060,8 @@ ag_status run_plan(ag_plan *pl, cudaStream_t s)
     AGB_CK(cudaEventRecord(c->evn0, s));
     if (need_near) {
         for (const NearGroup &g : pl->groups) {
-            AGB_CK(launch_near(exact, d, g, near_ptrs(pl, c->d_counters), 0, s));
+            AGB_CK(exact ? launch_near_exact(d, g, near_ptrs(pl, c->d_counters), s)
+                         : launch_near(d, g, near_ptrs(pl, c->d_counters), s));
             launches++;
         }
     }

@@ -144,6 +144,13 @@ __host__ inline void far_edge_multipliers(double p_max, bool p_exact, double rho
     *hi = (float)(1.0 + kh * 2 * u);    // floats above 1 are spaced 2^-23
 }
 
+// The same bound for near pairs, absolute, in bins: |t - D| for D <= FAR_T0 + 8.
+__host__ inline float near_edge_guard(double p_max, bool p_exact, double rho_ulps)
+{
+    const double d = (4.5 + rho_ulps) * ((double)FAR_T0 + 8.0) + (p_exact ? 1.0 : 2.0) * p_max;
+    return (float)(d * 1.0625 / 16777216.0);
+}
+
 // Streaming multiprocessors of the current device (launch sizing).
 int current_device_sms();
 
@@ -159,6 +166,7 @@ struct DevProblem {
     double cov_pos[3], cov_half_width, cov_barrier;
     int any_covalent;
     int report_collisions;             // 'map_receptor_interior off' (ag_problem)
+    float near_guard;                  // error bound (bins) of the canonical FP32 distance of a near pair
 
     // atoms in file order (FP64, centred)
     const double *x, *y, *z, *q, *vol, *solpar;

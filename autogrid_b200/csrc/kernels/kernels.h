@@ -19,22 +19,6 @@ struct NearPtrs {
     unsigned long long *counters;
 };
 
-struct NearSmem {
-    float4 pos[NB_CHUNK_MAX], a[NB_CHUNK_MAX], b[NB_CHUNK_MAX];
-    int meta[NB_CHUNK_MAX], idx[NB_CHUNK_MAX];
-    int hl[NB_CHUNK_MAX], nh;  // staged DS/D1 candidates (slots in this chunk), any order
-    // per warp: slots of the staged atoms near that warp's points, in staged order
-    unsigned short wl[NB_WARPS_MAX][NB_CHUNK_MAX];
-    float wbox[NB_WARPS_MAX][6];  // per warp: its points' box in frame bins (lo xyz, hi xyz)
-    float etab[NT_SMALL], sol[NT_SMALL];
-    // per thread: the running H-bond min/max of the MM maps (FP32 kernels;
-    // in shared memory, out of the pair loop's 80-register budget)
-    float hmin[NG_MM][NB_THREADS_MAX], hmax[NG_MM][NB_THREADS_MAX];
-    int seg_start[NB_SEGS_MAX], seg_off[NB_SEGS_MAX + 1];
-    int tcnt[NB_CHUNK_MAX / 32][32];  // staging by receptor type: per 32-candidate slice and type
-    int total;
-};
-
 struct NearInst {
     DevProblem p;
     NearGroup g;
@@ -82,8 +66,11 @@ cudaError_t launch_collisions(const DevProblem &p, long long lin0, long long lin
 // added into g_xyz [3N] (FP64); g_fmap [P] in FP32 or FP64.
 cudaError_t launch_fmap_adjoint(const DevProblem &p, const void *g_fmap, bool fp64, double *g_xyz, cudaStream_t s);
 int near_bricks(const DevProblem &p, int shape);
-cudaError_t launch_near(bool exact, const DevProblem &p, const NearGroup &g, const NearPtrs &ptr, int shape,
-                        cudaStream_t s, int bz0 = 0, int bz1 = -1);
+// FP32 (kernels/near_rows.cu; brick z-rows [bz0, bz1), bz1 < 0: through the
+// last) and the FP64 twin (kernels/near.cu).
+cudaError_t launch_near(const DevProblem &p, const NearGroup &g, const NearPtrs &ptr, cudaStream_t s, int bz0 = 0,
+                        int bz1 = -1);
+cudaError_t launch_near_exact(const DevProblem &p, const NearGroup &g, const NearPtrs &ptr, cudaStream_t s);
 // max_ng: the most maps any instance's group holds (picks the accumulator count)
 cudaError_t launch_near_batch(const NearInst *insts, const long long *unit_begin, int n_inst,
                               unsigned long long *counter, int shape, int ctas_per_sm, int max_ng, cudaStream_t s);
