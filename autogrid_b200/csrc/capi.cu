@@ -502,17 +502,23 @@ ag_status build_plan(ag_plan *pl, const ag_problem *p, cudaStream_t s, bool pipe
             pl->far_const = (float)p->invdielcal;
         }
     }
-    // far-field chunking: enough CTAs for ~8 waves per launch; a slab-pipelined
-    // one-shot run launches one slab of frames at a time, ~3 waves each
+    // far-field chunking: units of at least kFarMinChunk atoms, enough for 4
+    // waves of CTAs per launch; a slab-pipelined one-shot run launches one slab
+    // of frames at a time, 5 waves of at least half that.  (10,000 atoms, 127^3
+    // points: 2 and 8 waves took 10.04 ms as 4 do, 16 10.07 ms; one-shot, 3
+    // waves 11.08, 5 10.88, 8 10.97 ms.  1,800 atoms, 41^3 points: chunks of 512
+    // atoms 136 us, 256 147 us, 128 155 us, as a unit's table load and sums
+    // then weigh more.)
     const long long frames = pipelined ? (long long)frames_x(d.n1x) * frames_y(d.n1y) * (kSlabZ / FRAME_Z)
                                        : (long long)frames_x(d.n1x) * frames_y(d.n1y) * frames_z(d.n1z);
-    const int tile = 512;
     if (p->elec_map >= 0 && N > 0) {
+        constexpr int kFarMinChunk = 512, kFarQuantum = 64;  // both halves of a CTA take whole 32-atom blocks
         const long long sms = pl->ctx ? pl->ctx->sms : 148;
-        const long long target = pipelined ? sms * 3 * 3 : sms * 3 * 8;
+        const long long target = sms * FAR_CTAS_PER_SM * (pipelined ? 5 : 4);
+        const int least = pipelined ? kFarMinChunk / 2 : kFarMinChunk;
         int nch = (int)std::max(1LL, (target + frames - 1) / frames);
-        nch = std::min(nch, (N + tile - 1) / tile);
-        pl->chunk_atoms = ((N + nch - 1) / nch + tile - 1) / tile * tile;
+        nch = std::min(nch, (N + least - 1) / least);
+        pl->chunk_atoms = ((N + nch - 1) / nch + kFarQuantum - 1) / kFarQuantum * kFarQuantum;
         pl->n_chunks = (N + pl->chunk_atoms - 1) / pl->chunk_atoms;
     } else {
         pl->chunk_atoms = 0;
@@ -1139,7 +1145,7 @@ struct ag_batch {
     long long *d_far_begin = nullptr, *d_near_begin = nullptr;
     unsigned long long *d_counters = nullptr;  // kCounters: see its definition
     ag_tuning tune{};
-    int far_ctas_per_sm = 3, near_ctas_per_sm = 3;  // resident CTAs per SM of the persistent kernels
+    int far_ctas_per_sm = FAR_CTAS_PER_SM, near_ctas_per_sm = 3;  // resident CTAs per SM of the persistent kernels
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     ~ag_batch()
@@ -1154,13 +1160,20 @@ namespace {
 // Far-field work units of one instance with the given chunking.
 long long far_units(const FarArgs &a) { return (long long)a.nfx * a.nfy * a.nfz * ((a.n_atoms + a.chunk_atoms - 1) / std::max(1, a.chunk_atoms)); }
 
-ag_status batch_upload_far(ag_batch *b, bool chunked)
+// Atoms per far-field unit of an instance: all, or chunks of 2048 or 512.
+constexpr int kFarChunkings = 3;
+int far_chunk_atoms(int chunking, int n_atoms)
 {
-    // chunking: one unit per (frame, all atoms), or per (frame, 2048-atom chunk)
+    const int all = std::max(n_atoms, 1);
+    return chunking == 0 ? all : std::min(all, chunking == 1 ? 2048 : 512);
+}
+
+ag_status batch_upload_far(ag_batch *b, int chunking)
+{
     b->far_begin.assign(1, 0);
     for (size_t i = 0; i < b->far.size(); i++) {
         FarArgs &a = b->far[i];
-        a.chunk_atoms = chunked ? std::min(2048, std::max(a.n_atoms, 1)) : std::max(a.n_atoms, 1);
+        a.chunk_atoms = far_chunk_atoms(chunking, a.n_atoms);
         a.edge_words = far_edge_words(a.chunk_atoms);
         b->far_begin.push_back(b->far_begin.back() + (a.n_atoms > 0 ? far_units(a) : 0));
     }
@@ -1263,11 +1276,11 @@ ag_status batch_autotune(ag_batch *b)
     t = ag_tuning{};
     double best_far = 1e30, best_near = 1e30;
     int best_tile = 512, best_chunked = 0, best_shape = 0;
-    const int tiles[3] = {512, 256, 1024};
-    for (int chunked = 0; chunked < 2; chunked++) {
-        ag_status st = batch_upload_far(b, chunked != 0);
+    const int tiles[2] = {512, 1024};
+    for (int chunked = 0; chunked < kFarChunkings; chunked++) {
+        ag_status st = batch_upload_far(b, chunked);
         if (st != AG_OK) return st;
-        for (int ti = 0; ti < 3; ti++) {
+        for (int ti = 0; ti < 2; ti++) {
             double f = 0, n = 0;
             st = batch_time(b, tiles[ti], 0, &f, &n);
             if (st != AG_OK) return st;
@@ -1276,7 +1289,7 @@ ag_status batch_autotune(ag_batch *b)
             if (f < best_far) { best_far = f; best_tile = tiles[ti]; best_chunked = chunked; }
         }
     }
-    ag_status st = batch_upload_far(b, best_chunked != 0);
+    ag_status st = batch_upload_far(b, best_chunked);
     if (st != AG_OK) return st;
     for (int shape = 0; shape < 3; shape++) {
         double f = 0, n = 0;
@@ -1859,18 +1872,23 @@ static ag_status batch_create(ag_context *ctx, const ag_problem *const *problems
     b->red_begin.assign(1, 0);
     for (int i : order) {
         ag_plan *pl = b->plans[i].get();
-        // each instance's partial buffer must hold the chunked layout (at most ceil(N/2048) chunks)
-        const int max_chunks = std::max(1, (pl->dp.n_atoms + 2047) / 2048);
+        // each instance's buffers must hold every chunking of batch_upload_far
+        int max_chunks = 1;
+        for (int k = 0; k < kFarChunkings; k++) {
+            const int c = far_chunk_atoms(k, pl->dp.n_atoms);
+            max_chunks = std::max(max_chunks, (pl->dp.n_atoms + c - 1) / c);
+        }
         if (pl->dp.elec_map >= 0 && pl->dp.n_atoms > 0) {
             void *v = nullptr;
             AGB_CK(pl->bufs->ensure("far_partial", (size_t)max_chunks * (size_t)pl->dp.P * sizeof(float), &v));
             pl->far_partial = (float *)v;
             if (pl->far_mode != FAR_TAB_CONST) {
-                // edge bits for either chunking of batch_upload_far (2048-atom chunks or all atoms)
                 const int nframes = frames_x(pl->dp.n1x) * frames_y(pl->dp.n1y) * frames_z(pl->dp.n1z);
-                const int na = std::max(pl->dp.n_atoms, 1);
-                const size_t eb = std::max(far_edge_bits_bytes(max_chunks, std::min(2048, na), nframes),
-                                           far_edge_bits_bytes(1, na, nframes));
+                size_t eb = 0;
+                for (int k = 0; k < kFarChunkings; k++) {
+                    const int c = far_chunk_atoms(k, pl->dp.n_atoms);
+                    eb = std::max(eb, far_edge_bits_bytes((pl->dp.n_atoms + c - 1) / c, c, nframes));
+                }
                 AGB_CK(pl->bufs->ensure("edge_bits", eb, &v));
                 pl->edge_bits = (uint32_t *)v;
             }
@@ -1923,9 +1941,13 @@ static ag_status batch_create(ag_context *ctx, const ag_problem *const *problems
         st = batch_autotune(b.get());
         if (st != AG_OK) return st;
     } else {
-        st = batch_upload_far(b.get(), false);
-        if (st != AG_OK) return st;
         b->tune = ag_tuning{};
+        // 24 boxes of 1,000-12,000 atoms in one call: 512-atom chunks 23.6 ms,
+        // 2048 23.7 ms, whole instances 26.2 ms (the last units of a group of
+        // few boxes leave the GPU idle)
+        b->tune.far_chunked = 2;
+        st = batch_upload_far(b.get(), b->tune.far_chunked);
+        if (st != AG_OK) return st;
         b->tune.far_tile = 512;
         b->tune.near_shape = 0;
     }

@@ -6,10 +6,17 @@
 //                kernel, which evaluates them with exact bins.  Per pair:
 //                1 rsqrt (MUFU), packed FP32x2 arithmetic, one shared-memory
 //                table gather.  Atoms are streamed through shared memory in
-//                tiles; each thread keeps 8 grid points of one x-row in
+//                tiles; each thread keeps 16 grid points of two x-rows in
 //                registers (two-level summation: per-tile partial + total).
 //                The atom list is split into chunks for load balance; chunk
 //                partial sums land in far_partial[chunk][point].
+//                Bound by the shared-memory pipe: a random 32-lane gather
+//                takes 2.7 wavefronts, 6.1 ms for 10,000 atoms x 127^3 points;
+//                the kernel takes 6.79 ms (7.89 ms with 8 points per thread
+//                and guard bins compared by integer logic: 10.6 instructions
+//                per pair kept the issue slots 70% busy as well).  128
+//                registers and 2 CTAs per SM; 3 CTAs (80 registers) 7.50 ms,
+//                and 7.24 ms with the atom loop unrolled twice.
 // k_emap_reduce -- the e map: chunk partials added in fixed chunk order, then
 //                the near-field part the near kernel left in the map
 //                (deterministic; lets the far and near kernels run
@@ -24,6 +31,7 @@
 namespace agb {
 
 constexpr int EF_THREADS = 256;
+constexpr int EF_MIN_CTAS = FAR_CTAS_PER_SM;
 // float2 pairs of points per thread: 8 points of one x-row, FRAME_X wide
 constexpr int EF_PAIRS = FRAME_X / 8;
 
@@ -100,148 +108,184 @@ __device__ __forceinline__ size_t far_bits_base(const FarArgs &a, int f, int chu
     return ((size_t)chunk * (size_t)(a.nfx * a.nfy * a.nfz) + (size_t)f) * (size_t)a.edge_words * EF_THREADS;
 }
 
+// The far kernel works in units of 2^24 bins: a distance is then t * 2^-24, and
+// the product with edge * 2^-125, rounded toward zero into the subnormal
+// range, is the integer floor(t * edge) in the low bits of the float.
+// Scaling by powers of two is exact and rsqrt.approx repeats its mantissas
+// every two binades, so every t equals the near kernel's and the fix-up's.
+constexpr float FAR_DOWN = 5.9604644775390625e-08f;          // 2^-24
+constexpr float FAR_TINY_T2 = TINY_T2 * FAR_DOWN * FAR_DOWN;
+constexpr float FAR_EDGE_DOWN = 2.3509887016445750e-38f;     // 2^-125
+constexpr int EF_GROUP = EF_THREADS / 2;                     // threads that hold a frame's points
+
 // One work unit: frame `f` of one instance against atom chunk `chunk`.
 // The caller has loaded the instance's table into s_tab4 and synchronised.
-// Atom tile entries: frame-relative (Y, Z, X) in bins and w = q*coeff_estat*A_DIV,
-// in that order so that (Y, Z) arrive in an aligned register pair, the operand
-// of the packed y/z difference: with (X, Y, Z, w) the pair needed moves, and
-// the kernel took 8.20 against 7.89 ms for 127^3 points x 10,000 atoms.
-// The first NJ pairs of each thread hold the frame's x columns inside the box
-// (the rest is padding and is skipped), and a warp whose 4 rows or 2 planes
-// all lie past the box skips the pairs.
+// Each half of the CTA holds the whole frame and takes every other block of
+// 32 atoms: a thread holds 16 points, rows y and y + 4 of one plane with 8
+// points each, so that an atom's read, its x differences and the loop are
+// shared by 16 pairs.  (ROWS = 1: the box ends within the frame's first four
+// rows, and the second row is left out.)  The halves' sums meet in shared
+// memory at the end.
+// Atom tile entries: frame-relative (Y, Z, X) * 2^-24 in bins and
+// w = q*coeff_estat*A_DIV * 2^-24.
+// The first NJ pairs of each row hold the frame's x columns inside the box
+// (the rest is padding and is skipped), and a warp whose 2 planes lie past the
+// box skips the pairs.
 //
 // Table bins (FAR_TAB_TABLE).  Each pair's table value is T[floor(t*edge_lo)];
 // a pair whose second guard bin floor(t*edge_hi) differs lies within the FP32
-// error bound of a bin edge.  Each thread records one bit per atom with such
-// a pair among its own, one 32-bit word per 32 atoms, in a.edge_bits; the
-// fix-up kernel (k_far_fixup) resolves those pairs afterwards.
+// error bound of a bin edge.  With n = -floor(t*edge_lo) in the subnormal
+// range, RZ(t*edge_hi + (E + n)) adds the difference of the two bins to E
+// exactly, so the guard of a row's 8 pairs is 2 packed operations per 2 pairs
+// and one test at the end.  Each row records one bit per atom with such a pair
+// among its own, one 32-bit word per 32 atoms, in a.edge_bits; the fix-up
+// kernel (k_far_fixup) resolves those pairs afterwards.
 // CLAMP: t is clamped half a bin past the last bin; without it the table
 // extends past bin NDIEL-1 (repeating that bin's value) to a length that
 // covers every distance of the instance, which saves the per-pair clamp.
-template <int TILE, int MODE, int NJ, bool CLAMP>
+template <int TILE, int MODE, int NJ, int ROWS, bool CLAMP>
 __device__ __forceinline__ void far_unit_n(const FarArgs &a, int f, int chunk, const float4 *s_tab4, float4 *s_atom)
 {
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31, v = (tid >> 5) & 3, half = tid / EF_GROUP;
     const int fx = f % a.nfx, fy = (f / a.nfx) % a.nfy, fz = f / (a.nfx * a.nfy);
     const int ox = fx * FRAME_X, oy = fy * FRAME_Y, oz = fz * FRAME_Z;
     // frame origin in bins, exactly (ox-nex)*spacing*A_DIV as the reference forms c (main.cpp:2859)
     const double X0 = frame_origin_bins(ox, a.nex, a.spacing_adiv);
     const double Y0 = frame_origin_bins(oy, a.ney, a.spacing_adiv);
     const double Z0 = frame_origin_bins(oz, a.nez, a.spacing_adiv);
-    const FarLane L = far_lane(a, tid, oy, oz);
-    const float py = frame_point_coord(L.ty, a.spacing_adiv);
-    const float pz = frame_point_coord(L.tz, a.spacing_adiv);
+    // lane footprint 4x4x2 (fewest table bank conflicts): x = tx + 8j and tx + 8j + 4
+    const int tx = lane & 3, ty = (lane >> 2) & 3, tz = (lane >> 4) + 2 * v;
+    const bool warp_in = oz + 2 * v < a.n1z;
+    const float npz = -frame_point_coord(tz, a.spacing_adiv) * FAR_DOWN;
+    const float2 npy = make_float2(-frame_point_coord(ty, a.spacing_adiv) * FAR_DOWN,
+                                   -frame_point_coord(ty + 4, a.spacing_adiv) * FAR_DOWN);
     float2 npx[NJ];
 #pragma unroll
     for (int j = 0; j < NJ; j++)
-        npx[j] = make_float2(-frame_point_coord(L.tx + 8 * j, a.spacing_adiv),
-                             -frame_point_coord(L.tx + 8 * j + 4, a.spacing_adiv));
-    const float2 npyz = make_float2(-py, -pz);
-    float2 tot[NJ];
+        npx[j] = make_float2(-frame_point_coord(tx + 8 * j, a.spacing_adiv) * FAR_DOWN,
+                             -frame_point_coord(tx + 8 * j + 4, a.spacing_adiv) * FAR_DOWN);
+    float2 tot[ROWS][NJ];
 #pragma unroll
-    for (int j = 0; j < NJ; j++) tot[j] = make_float2(0.f, 0.f);
+    for (int r = 0; r < ROWS; r++)
+#pragma unroll
+        for (int j = 0; j < NJ; j++) tot[r][j] = make_float2(0.f, 0.f);
 
-    // 32-bit shared address of the table, pre-biased so that the bit pattern of
-    // (t + 2^23) rounded toward zero indexes it directly:
-    // bits(t + 2^23) = 0x4B000000 + floor(t) for 0 <= t < 2^23.
-    const uint32_t tab_base = (uint32_t)__cvta_generic_to_shared(s_tab4) - (MAGIC_BITS << 2);
-    const float2 lom = make_float2(a.edge_lo, a.edge_lo), him = make_float2(a.edge_hi, a.edge_hi);
-    uint32_t *bits = (MODE == FAR_TAB_TABLE && a.edge_bits) ? a.edge_bits + far_bits_base(a, f, chunk) + tid : nullptr;
+    const uint32_t tab_base = (uint32_t)__cvta_generic_to_shared(s_tab4);
+    const float2 nlom = make_float2(-a.edge_lo * FAR_EDGE_DOWN, -a.edge_lo * FAR_EDGE_DOWN);
+    const float2 him = make_float2(a.edge_hi * FAR_EDGE_DOWN, a.edge_hi * FAR_EDGE_DOWN);
+    uint32_t *bits = (MODE == FAR_TAB_TABLE && a.edge_bits) ? a.edge_bits + far_bits_base(a, f, chunk) + 64 * v + lane : nullptr;
 
     const int a_begin = chunk * a.chunk_atoms;
     const int a_end = min(a.n_atoms, a_begin + a.chunk_atoms);
     for (int a0 = a_begin; a0 < a_end; a0 += TILE) {
         const int na = min(TILE, a_end - a0);
         __syncthreads();
-        for (int i = tid; i < TILE; i += EF_THREADS) {
-            float4 v;
-            if (i < na) {
-                const int at = a0 + i;
-                v.z = frame_atom_coord(__ldg(a.ax128 + at), X0);
-                v.x = frame_atom_coord(__ldg(a.ay128 + at), Y0);
-                v.y = frame_atom_coord(__ldg(a.az128 + at), Z0);
-                v.w = __ldg(a.qw + at);
-            } else {
-                v = make_float4(0.f, 0.f, 0.f, 0.f);  // never read: the pair loops stop at na
-            }
-            s_atom[i] = v;
+        for (int i = tid; i < na; i += EF_THREADS) {
+            const int at = a0 + i;
+            float4 t;
+            t.z = frame_atom_coord(__ldg(a.ax128 + at), X0) * FAR_DOWN;
+            t.x = frame_atom_coord(__ldg(a.ay128 + at), Y0) * FAR_DOWN;
+            t.y = frame_atom_coord(__ldg(a.az128 + at), Z0) * FAR_DOWN;
+            t.w = __ldg(a.qw + at) * FAR_DOWN;
+            s_atom[i] = t;
         }
         __syncthreads();
-        if (!L.warp_in) continue;
-        float2 acc[NJ];
+        if (!warp_in) continue;
+        float2 acc[ROWS][NJ];
 #pragma unroll
-        for (int j = 0; j < NJ; j++) acc[j] = make_float2(0.f, 0.f);
-        if (MODE == FAR_TAB_CONST) {
-            const float2 fT0 = make_float2(FAR_T0, FAR_T0);
-#pragma unroll 2
-            for (int i = 0; i < na; i++) {
-                const float4 A = s_atom[i];
-                const float2 dyz = __fadd2_rn(make_float2(A.x, A.y), npyz);
-                const float s = __fmaf_rn(dyz.x, dyz.x, __fmaf_rn(dyz.y, dyz.y, TINY_T2));
-                const float2 s2 = make_float2(s, s);
-                const float2 ax2 = make_float2(A.z, A.z);
-                const float2 q2 = make_float2(A.w, A.w);
+        for (int r = 0; r < ROWS; r++)
+#pragma unroll
+            for (int j = 0; j < NJ; j++) acc[r][j] = make_float2(0.f, 0.f);
+        for (int ib = 32 * half; ib < na; ib += 64) {
+            const int nb = min(32, na - ib);
+            uint32_t hist[ROWS];
+#pragma unroll
+            for (int r = 0; r < ROWS; r++) hist[r] = 0;
+#pragma unroll 1
+            for (int ii = 0; ii < nb; ii++) {
+                const float4 A = s_atom[ib + ii];
+                const float2 dy = __fadd2_rn(make_float2(A.x, A.x), npy);
+                const float dz = __fadd_rn(A.y, npz);
+                const float zz = __fmaf_rn(dz, dz, FAR_TINY_T2);
+                const float2 s = __ffma2_rn(dy, dy, make_float2(zz, zz));
+                const float2 ax2 = make_float2(A.z, A.z), q2 = make_float2(A.w, A.w);
+                float2 E[ROWS];
 #pragma unroll
                 for (int j = 0; j < NJ; j++) {
                     const float2 dx = __fadd2_rn(ax2, npx[j]);
-                    const float2 t2 = __ffma2_rn(dx, dx, s2);
-                    const float2 rs = make_float2(rsqrt_approx(t2.x), rsqrt_approx(t2.y));
-                    const float2 t = __fmul2_rn(t2, rs);
-                    const float T0 = t.x < fT0.x ? 0.f : a.tab_const;
-                    const float T1 = t.y < fT0.y ? 0.f : a.tab_const;
-                    const float2 wv = __fmul2_rn(q2, rs);
-                    acc[j] = __ffma2_rn(wv, make_float2(T0, T1), acc[j]);
-                }
-            }
-        } else {
-            const float2 tmax = make_float2(FAR_CLAMP_T, FAR_CLAMP_T);
-            for (int ib = 0; ib < na; ib += 32) {
-                const int nb = min(32, na - ib);
-                uint32_t hist = 0;
-#pragma unroll 2
-                for (int ii = 0; ii < nb; ii++) {
-                    const float4 A = s_atom[ib + ii];
-                    const float2 dyz = __fadd2_rn(make_float2(A.x, A.y), npyz);
-                    const float s = __fmaf_rn(dyz.x, dyz.x, __fmaf_rn(dyz.y, dyz.y, TINY_T2));
-                    const float2 s2 = make_float2(s, s);
-                    const float2 ax2 = make_float2(A.z, A.z);
-                    const float2 q2 = make_float2(A.w, A.w);
-                    uint32_t edge = 0;
 #pragma unroll
-                    for (int j = 0; j < NJ; j++) {
-                        const float2 dx = __fadd2_rn(ax2, npx[j]);
-                        const float2 t2 = __ffma2_rn(dx, dx, s2);
+                    for (int r = 0; r < ROWS; r++) {
+                        const float sr = r ? s.y : s.x;
+                        const float2 t2 = __ffma2_rn(dx, dx, make_float2(sr, sr));
                         const float2 rs = make_float2(rsqrt_approx(t2.x), rsqrt_approx(t2.y));
                         float2 t = __fmul2_rn(t2, rs);
-                        if (CLAMP) t = make_float2(fminf(t.x, tmax.x), fminf(t.y, tmax.y));
-                        float2 lo, hi;
-                        far_guard_bins(t, lom, him, lo, hi);
-                        edge |= (__float_as_uint(lo.x) ^ __float_as_uint(hi.x)) |
-                                (__float_as_uint(lo.y) ^ __float_as_uint(hi.y));
-                        const float T0 = lds_f32(tab_base + (__float_as_uint(lo.x) << 2));
-                        const float T1 = lds_f32(tab_base + (__float_as_uint(lo.y) << 2));
-                        const float2 wv = __fmul2_rn(q2, rs);
-                        acc[j] = __ffma2_rn(wv, make_float2(T0, T1), acc[j]);
+                        if (MODE == FAR_TAB_CONST) {
+                            const float T0 = t.x < FAR_T0 * FAR_DOWN ? 0.f : a.tab_const;
+                            const float T1 = t.y < FAR_T0 * FAR_DOWN ? 0.f : a.tab_const;
+                            acc[r][j] = __ffma2_rn(__fmul2_rn(q2, rs), make_float2(T0, T1), acc[r][j]);
+                            continue;
+                        }
+                        if (CLAMP) t = make_float2(fminf(t.x, FAR_CLAMP_T * FAR_DOWN), fminf(t.y, FAR_CLAMP_T * FAR_DOWN));
+                        const float2 nlo = __fmul2_rz(t, nlom);
+                        E[r] = __ffma2_rz(t, him, j ? __fadd2_rn(E[r], nlo) : nlo);
+                        // the sign bit leaves with the shift
+                        const float T0 = lds_f32(tab_base + (__float_as_uint(nlo.x) << 2));
+                        const float T1 = lds_f32(tab_base + (__float_as_uint(nlo.y) << 2));
+                        acc[r][j] = __ffma2_rn(__fmul2_rn(q2, rs), make_float2(T0, T1), acc[r][j]);
                     }
-                    hist = (hist << 1) | (edge ? 1u : 0u);
                 }
-                if (bits) bits[(size_t)((a0 - a_begin + ib) >> 5) * EF_THREADS] = hist << (32 - nb);  // atom k at bit 31-k
+                if (MODE == FAR_TAB_TABLE)
+#pragma unroll
+                    for (int r = 0; r < ROWS; r++)
+                        hist[r] = (hist[r] << 1) | ((__float_as_uint(E[r].x) | __float_as_uint(E[r].y)) ? 1u : 0u);
             }
+            if (MODE == FAR_TAB_TABLE && bits)
+#pragma unroll
+                for (int r = 0; r < ROWS; r++)  // atom k at bit 31-k
+                    bits[(size_t)((a0 - a_begin + ib) >> 5) * EF_THREADS + 32 * r] = hist[r] << (32 - nb);
         }
 #pragma unroll
-        for (int j = 0; j < NJ; j++) tot[j] = __fadd2_rn(tot[j], acc[j]);
+        for (int r = 0; r < ROWS; r++)
+#pragma unroll
+            for (int j = 0; j < NJ; j++) tot[r][j] = __fadd2_rn(tot[r][j], acc[r][j]);
     }
 
-    const int iy = oy + L.ty, iz = oz + L.tz;
-    if (iy < a.n1y && iz < a.n1z) {
-        float *out = a.partial + (size_t)chunk * (size_t)a.P + ((size_t)iz * a.n1y + iy) * (size_t)a.n1x;
+    // the second half's sums through the atom tile, 8 KB
+    static_assert(TILE * sizeof(float4) >= 16 * EF_GROUP * sizeof(float), "the tile holds one half's sums");
+    float *ex = (float *)s_atom + (tid & (EF_GROUP - 1));
+    __syncthreads();
+    if (half == 1)
 #pragma unroll
-        for (int j = 0; j < NJ; j++) {
-            const int ix0 = ox + L.tx + 8 * j, ix1 = ix0 + 4;
-            if (ix0 < a.n1x) out[ix0] = tot[j].x;
-            if (ix1 < a.n1x) out[ix1] = tot[j].y;
+        for (int r = 0; r < ROWS; r++)
+#pragma unroll
+            for (int j = 0; j < NJ; j++) {
+                ex[(8 * r + 2 * j) * EF_GROUP] = tot[r][j].x;
+                ex[(8 * r + 2 * j + 1) * EF_GROUP] = tot[r][j].y;
+            }
+    __syncthreads();
+    if (half == 0 && oz + tz < a.n1z)
+#pragma unroll
+        for (int r = 0; r < ROWS; r++) {
+            const int iy = oy + ty + 4 * r, iz = oz + tz;
+            if (iy >= a.n1y) continue;
+            float *out = a.partial + (size_t)chunk * (size_t)a.P + ((size_t)iz * a.n1y + iy) * (size_t)a.n1x;
+#pragma unroll
+            for (int j = 0; j < NJ; j++) {
+                const int ix0 = ox + tx + 8 * j, ix1 = ix0 + 4;
+                if (ix0 < a.n1x) out[ix0] = tot[r][j].x + ex[(8 * r + 2 * j) * EF_GROUP];
+                if (ix1 < a.n1x) out[ix1] = tot[r][j].y + ex[(8 * r + 2 * j + 1) * EF_GROUP];
+            }
         }
-    }
+}
+
+// One or two rows per thread (CTA-uniform: only a box's last y frame can end
+// within its first four rows).
+template <int TILE, int MODE, int NJ, bool CLAMP>
+__device__ __forceinline__ void far_unit_r(const FarArgs &a, int f, int chunk, const float4 *s_tab4, float4 *s_atom)
+{
+    const int oy = ((f / a.nfx) % a.nfy) * FRAME_Y;
+    if (oy + 4 < a.n1y) far_unit_n<TILE, MODE, NJ, 2, CLAMP>(a, f, chunk, s_tab4, s_atom);
+    else far_unit_n<TILE, MODE, NJ, 1, CLAMP>(a, f, chunk, s_tab4, s_atom);
 }
 
 // The unit with as many x pairs as the frame has columns inside the box
@@ -252,10 +296,10 @@ __device__ __forceinline__ void far_unit(const FarArgs &a, int f, int chunk, con
 {
     static_assert(EF_PAIRS == 4, "x-pair dispatch below");
     const int nj = (a.n1x - (f % a.nfx) * FRAME_X + 7) / 8;
-    if (nj >= 4) far_unit_n<TILE, MODE, 4, CLAMP>(a, f, chunk, s_tab4, s_atom);
-    else if (nj == 3) far_unit_n<TILE, MODE, 3, CLAMP>(a, f, chunk, s_tab4, s_atom);
-    else if (nj == 2) far_unit_n<TILE, MODE, 2, CLAMP>(a, f, chunk, s_tab4, s_atom);
-    else far_unit_n<TILE, MODE, 1, CLAMP>(a, f, chunk, s_tab4, s_atom);
+    if (nj >= 4) far_unit_r<TILE, MODE, 4, CLAMP>(a, f, chunk, s_tab4, s_atom);
+    else if (nj == 3) far_unit_r<TILE, MODE, 3, CLAMP>(a, f, chunk, s_tab4, s_atom);
+    else if (nj == 2) far_unit_r<TILE, MODE, 2, CLAMP>(a, f, chunk, s_tab4, s_atom);
+    else far_unit_r<TILE, MODE, 1, CLAMP>(a, f, chunk, s_tab4, s_atom);
 }
 
 template <int TILE>
@@ -271,7 +315,7 @@ __device__ __forceinline__ void far_dispatch(const FarArgs &a, int f, int chunk,
 // launch, so a grid whose last x frame is full compiles to the full-frame unit
 // alone.
 template <int TILE, int NJ_LAST, bool CLAMP>
-__global__ void __launch_bounds__(EF_THREADS, 3) k_emap_far(FarArgs a)
+__global__ void __launch_bounds__(EF_THREADS, EF_MIN_CTAS) k_emap_far(FarArgs a)
 {
     extern __shared__ float4 ef_smem[];
     float4 *s_tab4 = ef_smem;                     // a.tab_len floats
@@ -281,11 +325,11 @@ __global__ void __launch_bounds__(EF_THREADS, 3) k_emap_far(FarArgs a)
     const int f = a.frame0 + blockIdx.x;
     const bool last = NJ_LAST < EF_PAIRS && f % a.nfx == a.nfx - 1;
     if (a.tab_mode == FAR_TAB_CONST) {
-        if (last) far_unit_n<TILE, FAR_TAB_CONST, NJ_LAST, true>(a, f, blockIdx.y, s_tab4, s_atom);
-        else far_unit_n<TILE, FAR_TAB_CONST, EF_PAIRS, true>(a, f, blockIdx.y, s_tab4, s_atom);
+        if (last) far_unit_r<TILE, FAR_TAB_CONST, NJ_LAST, true>(a, f, blockIdx.y, s_tab4, s_atom);
+        else far_unit_r<TILE, FAR_TAB_CONST, EF_PAIRS, true>(a, f, blockIdx.y, s_tab4, s_atom);
     } else {
-        if (last) far_unit_n<TILE, FAR_TAB_TABLE, NJ_LAST, CLAMP>(a, f, blockIdx.y, s_tab4, s_atom);
-        else far_unit_n<TILE, FAR_TAB_TABLE, EF_PAIRS, CLAMP>(a, f, blockIdx.y, s_tab4, s_atom);
+        if (last) far_unit_r<TILE, FAR_TAB_TABLE, NJ_LAST, CLAMP>(a, f, blockIdx.y, s_tab4, s_atom);
+        else far_unit_r<TILE, FAR_TAB_TABLE, EF_PAIRS, CLAMP>(a, f, blockIdx.y, s_tab4, s_atom);
     }
 }
 
@@ -557,7 +601,7 @@ __global__ void __launch_bounds__(EF_THREADS) k_far_fixup_batch(const FarArgs *_
 // instance (instances ordered by decreasing work) and never wait on each other.
 // The dynamic shared memory holds the longest table of the batch and a tile.
 template <int TILE>
-__global__ void __launch_bounds__(EF_THREADS, 3)
+__global__ void __launch_bounds__(EF_THREADS, EF_MIN_CTAS)
 k_emap_far_batch(const FarArgs *__restrict__ insts, const long long *__restrict__ unit_begin, int n_inst,
                  unsigned long long *__restrict__ counter, int max_tab_len)
 {
@@ -767,10 +811,9 @@ cudaError_t prepare_far_kernels()
         cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FixSmem));
         if (e != cudaSuccess) return e;
     }
-    const void *batch[] = {(const void *)k_emap_far_batch<256>, (const void *)k_emap_far_batch<512>,
-                           (const void *)k_emap_far_batch<1024>};
-    const int tiles[] = {256, 512, 1024};
-    for (int k = 0; k < 3; k++) {
+    const void *batch[] = {(const void *)k_emap_far_batch<512>, (const void *)k_emap_far_batch<1024>};
+    const int tiles[] = {512, 1024};
+    for (int k = 0; k < 2; k++) {
         cudaError_t e = cudaFuncSetAttribute(batch[k], cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)far_smem_bytes(tiles[k], FAR_TAB_MAX));
         if (e != cudaSuccess) return e;
@@ -799,7 +842,6 @@ cudaError_t launch_emap_far_batch(const FarArgs *insts, const long long *unit_be
                                   cudaStream_t s)
 {
     if (max_tab_len < 0 || max_tab_len > FAR_TAB_MAX || max_tab_len % 4) return cudaErrorInvalidValue;
-    if (tile == 256) return far_batch_t<256>(insts, unit_begin, n_inst, counter, ctas_per_sm, max_tab_len, s);
     if (tile == 1024) return far_batch_t<1024>(insts, unit_begin, n_inst, counter, ctas_per_sm, max_tab_len, s);
     return far_batch_t<512>(insts, unit_begin, n_inst, counter, ctas_per_sm, max_tab_len, s);
 }

@@ -26,6 +26,8 @@ struct NearInst {
 };
 
 
+// Resident CTAs per SM the far kernels are compiled for (launch sizing).
+constexpr int FAR_CTAS_PER_SM = 2;
 size_t far_smem_bytes(int tile, int tab_len);
 // Dynamic shared-memory limits of the far kernels on the current device.
 cudaError_t prepare_far_kernels();

@@ -1,0 +1,52 @@
+"""Far-field kernel units at the edges of their tiling: boxes whose last frame
+holds 1-4 or more rows and columns, atom counts around the 32-atom blocks that
+the two halves of a CTA share out, the clamped table and a constant dielectric.
+
+The e map is compared with the FP64 oracle.  A point's sum is built from runs
+of at most 256 terms, so rounding stays below 255 + 8 units of 2^-24 of the sum
+of the terms' magnitudes (8: the terms' own roundings); a pair in a wrong table
+bin is off by a thousandth of its term, more than that for the small counts.
+"""
+import numpy as np
+import pytest
+
+from conftest import make_case
+
+pytestmark = pytest.mark.gpu
+
+BOXES = [(2, 2, 2), (8, 4, 6), (30, 8, 8), (32, 10, 2), (40, 14, 10), (56, 6, 16)]
+
+
+def _bound(prob):
+    a, s = prob.arrays, prob.scalars
+    ax = [(np.arange(n) - (n - 1) // 2) * s["spacing"] for n in prob.n1]
+    z, y, x = np.meshgrid(ax[2], ax[1], ax[0], indexing="ij")
+    pts = np.stack([x, y, z], -1).reshape(-1, 3)
+    c, q = a["coord"].reshape(-1, 3), a["charge"]
+    out = np.zeros(len(pts))
+    for i in range(len(q)):
+        r = np.sqrt(((c[i] - pts) ** 2).sum(1))
+        k = np.minimum((r * 128).astype(int), 8191)
+        T = a["r_epsilon_fn"][k] if s["dddiel"] else s["invdielcal"]
+        out += np.abs(q[i]) * T * s["coeff_estat"] / np.maximum(r, 0.5)
+    return 263 * 2.0 ** -24 * out + 1e-30
+
+
+@pytest.mark.parametrize("mode", ["table", "clamp", "const"])
+@pytest.mark.parametrize("n_atoms", [40, 65, 513])
+@pytest.mark.parametrize("npts", BOXES)
+def test_e_map_against_oracle(tmp_path, gpu_ctx, npts, n_atoms, mode):
+    from oracle.oracle import oracle_points
+    kw = dict(radius=160.0) if mode == "clamp" else {}
+    _, prob = make_case(tmp_path, "far", n_atoms, npts, seed=sum(npts) + n_atoms, ligand_types=["C"],
+                        dielectric=40.0 if mode == "const" else -0.1465, **kw)
+    e = prob.scalars["elec_map"]
+    ref, flags = oracle_points(prob)
+    got = gpu_ctx.compute(prob, "fp32").reshape(prob.n_maps, -1)[e]
+    off = np.abs(got - ref[e]) > _bound(prob)
+    assert not (off & (flags == 0)).any()
+    plan = gpu_ctx.plan(prob)
+    plan.run()
+    again = plan.download().reshape(prob.n_maps, -1)[e]
+    assert not ((np.abs(again - ref[e]) > _bound(prob)) & (flags == 0)).any()
+    plan.close()
