@@ -262,9 +262,11 @@ struct ag_plan {
     int far_mode = FAR_TAB_TABLE;        // how k_emap_far obtains far table values (FarArgs::tab_mode)
     int tab_len = AG_NDIEL, far_clamp = 1;  // shared-memory far table (FarArgs::tab_len, clamp)
     float far_const = 0.f;
+    double max_bins = 0.0;               // at least the largest atom-to-point distance, in bins
     double constriction_cutoff = 7.5;
     float *maps32 = nullptr;
     double *maps64 = nullptr;
+    double *emap64_partial = nullptr;  // FP64 e map: sums per atom chunk
     double *cov = nullptr;
     float *far_partial = nullptr;
     uint32_t *edge_bits = nullptr;     // far-field bin guard: per (thread, atom) edge bits (FarArgs::edge_bits)
@@ -478,6 +480,7 @@ ag_status build_plan(ag_plan *pl, const ag_problem *p, cudaStream_t s, bool pipe
             dmax2 = std::max(dmax2, d2);
         }
         const double tmax = std::sqrt(dmax2) * AG_A_DIV * (1.0 + 1.0e-5) + 8.0;
+        pl->max_bins = tmax;
         if (tmax < (double)FAR_TAB_MAX - 4.0) {
             pl->far_clamp = 0;
             pl->tab_len = ((int)std::ceil(tmax) + 4) / 4 * 4;
@@ -791,6 +794,10 @@ ag_status build_plan(ag_plan *pl, const ag_problem *p, cudaStream_t s, bool pipe
         AGB_CK(B->ensure("maps64", n_out * P * sizeof(double), &v));
         pl->maps64 = (double *)v;
         pl->maps32 = nullptr;
+        if (d.elec_map >= 0 && emap_exact_chunks(d) > 1) {
+            AGB_CK(B->ensure("emap64_partial", (size_t)emap_exact_chunks(d) * P * sizeof(double), &v));
+            pl->emap64_partial = (double *)v;
+        }
     } else {
         AGB_CK(B->ensure("maps32", n_out * P * sizeof(float), &v));
         pl->maps32 = (float *)v;
@@ -1026,8 +1033,8 @@ ag_status run_plan(ag_plan *pl, cudaStream_t s)
     AGB_CK(cudaEventRecord(c->ev0, s));
     const bool far = !exact && d.elec_map >= 0 && pl->n_chunks > 0;
     if (d.elec_map >= 0 && exact) {
-        AGB_CK(launch_emap_exact(d, pl->maps64 + (size_t)d.elec_map * d.P, s));
-        launches++;
+        AGB_CK(launch_emap_exact(d, pl->max_bins, pl->maps64 + (size_t)d.elec_map * d.P, pl->emap64_partial, s));
+        launches += pl->emap64_partial ? 2 : 1;
     }
     // far field on the side stream, concurrent with the near-field kernel (or,
     // with opts.serial, before it on s)

@@ -67,6 +67,17 @@ __device__ __forceinline__ float sqrt_approx(float x)
     return y;
 }
 
+// 1/sqrt(x) in FP64, x > 0 normal, within a few ulp: the hardware's
+// approximation (relative error e/2 of at most 2^-20) and one Householder
+// iteration of third order, y (1 + e/2 + 3 e^2/8 + O(e^3)) with e = 1 - x y^2.
+__device__ __forceinline__ double rsqrt_f64(double x)
+{
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = __fma_rn(-__dmul_rn(x, y), y, 1.0);
+    return __fma_rn(__dmul_rn(y, e), __fma_rn(0.375, e, 0.5), y);
+}
+
 // The far kernel's distance (in bins) of a pair, from frame-relative FP32
 // inputs.  Written with explicit round-to-nearest intrinsics so no contraction
 // or reassociation can make two call sites differ.

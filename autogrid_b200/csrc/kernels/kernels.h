@@ -54,7 +54,10 @@ struct ReduceInst {
 cudaError_t launch_emap_reduce(const ReduceInst *insts, const long long *begin, int n, long long total,
                                cudaStream_t s);
 cudaError_t launch_emap_reduce_range(const ReduceInst &r, long long lin0, long long lin1, cudaStream_t s);
-cudaError_t launch_emap_exact(const DevProblem &p, double *emap, cudaStream_t s);
+// max_bins: at least the largest distance (bins) of an atom to a point;
+// partial: emap_exact_chunks(p) * P doubles when there are several chunks.
+int emap_exact_chunks(const DevProblem &p);
+cudaError_t launch_emap_exact(const DevProblem &p, double max_bins, double *emap, double *partial, cudaStream_t s);
 cudaError_t launch_covalent(const DevProblem &p, double *cov, cudaStream_t s);
 cudaError_t launch_distance_maps(const DevProblem &p, double cutoff, float *fmap32, float *cmap32, double *fmap64,
                                  double *cmap64, cudaStream_t s);

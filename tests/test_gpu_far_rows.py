@@ -50,3 +50,30 @@ def test_e_map_against_oracle(tmp_path, gpu_ctx, npts, n_atoms, mode):
     again = plan.download().reshape(prob.n_maps, -1)[e]
     assert not ((np.abs(again - ref[e]) > _bound(prob)) & (flags == 0)).any()
     plan.close()
+
+
+@pytest.mark.parametrize("mode", ["table", "beyond_256A", "const"])
+@pytest.mark.parametrize("npts,n_atoms", [((2, 2, 2), 3), ((14, 8, 6), 300), ((16, 6, 8), 257), ((34, 18, 4), 1100)])
+def test_fp64_e_map(tmp_path, gpu_ctx, npts, n_atoms, mode):
+    """The FP64 twin's bricks, atom chunks and fixed-point bins, against the
+    nested hypot in numpy; points with a pair within 1e-9 bins of an edge are
+    left out (the two hypots may differ there), and the rest agrees to the
+    rounding of the sums."""
+    kw = dict(radius=300.0) if mode == "beyond_256A" else {}
+    _, prob = make_case(tmp_path, "far64", max(n_atoms, 20), npts, seed=sum(npts) + n_atoms, ligand_types=["C"],
+                        dielectric=40.0 if mode == "const" else -0.1465, **kw)
+    a, s = prob.arrays, prob.scalars
+    ax = [(np.arange(n) - (n - 1) // 2) * s["spacing"] for n in prob.n1]
+    z, y, x = (v.ravel() for v in np.meshgrid(ax[2], ax[1], ax[0], indexing="ij"))
+    c, q = a["coord"].reshape(-1, 3), a["charge"]
+    ref, size, tie = np.zeros(x.size), np.zeros(x.size), np.zeros(x.size, bool)
+    for i in range(len(q)):
+        r = np.maximum(np.hypot(c[i, 0] - x, np.hypot(c[i, 1] - y, c[i, 2] - z)), 1e-6)
+        tie |= np.abs(r * 128 - np.rint(r * 128)) < 1e-9
+        f = a["r_epsilon_fn"][np.minimum((r * 128).astype(int), 8191)] if s["dddiel"] else s["invdielcal"]
+        term = q[i] / np.maximum(r, 0.5) * f * s["coeff_estat"]
+        ref += term
+        size += np.abs(term)
+    got = gpu_ctx.compute(prob, "fp64").reshape(prob.n_maps, -1)[s["elec_map"]]
+    free = ~tie if s["dddiel"] else slice(None)
+    assert (np.abs(got - ref) <= 1e-12 * size + 1e-300)[free].all()
