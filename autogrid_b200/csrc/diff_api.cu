@@ -81,6 +81,8 @@ struct ag_diff {
     double *d_rv = nullptr, *d_rv2 = nullptr, *d_grad = nullptr;
     int *d_meta = nullptr, *d_h = nullptr, *d_cell_start = nullptr, *d_cell_atoms = nullptr;
     int *d_ch = nullptr, *d_mmarg = nullptr;
+    float *d_epart = nullptr;  // FP32 e map: sums per atom chunk
+    cudaTextureObject_t eps_tex = 0;  // the same table as a texture (FP32 e map)
     void *d_vdw = nullptr, *d_sol = nullptr, *d_eps = nullptr, *d_maps = nullptr, *d_gmaps = nullptr;
     cudaEvent_t ev[6] = {};
     float fwd_ms = 0, ch_ms = 0, bwd_ms = 0;
@@ -92,6 +94,7 @@ struct ag_diff {
     ~ag_diff()
     {
         cudaSetDevice(device);
+        if (eps_tex) cudaDestroyTextureObject(eps_tex);
         for (void *p : allocs) cudaFree(p);
         for (auto &e : ev)
             if (e) cudaEventDestroy(e);
@@ -446,6 +449,10 @@ ag_status ag_diff_create_batch(ag_context *ctx, const ag_problem *p, const ag_op
     DF_CK(d->alloc(&d->d_ch, (size_t)d->P * K));
     DF_CK(d->alloc(&d->d_mmarg, 2 * (size_t)n_mm * d->P * K));
     DF_CK(d->alloc(&d->d_grad, 10 * NK));
+    if (!d->fp64 && d->elec >= 0) {
+        DF_CK(prepare_elin());
+        if (elin_chunks(A) > 1) DF_CK(d->alloc(&d->d_epart, (size_t)elin_chunks(A) * d->P * K));
+    }
     unsigned char *mp = nullptr;
     DF_CK(d->alloc(&mp, d->map_bytes())); d->d_maps = mp;
     DF_CK(cudaMemcpy(d->d_vol, p->vol, N * sizeof(double), cudaMemcpyHostToDevice));
@@ -468,6 +475,16 @@ ag_status ag_diff_create_batch(ag_context *ctx, const ag_problem *p, const ag_op
         std::vector<R2<float>> sol, eps;
         build_tables(p, sol, eps);
         DF_CK(put(&d->d_vdw, rows, d.get())); DF_CK(put(&d->d_sol, sol, d.get())); DF_CK(put(&d->d_eps, eps, d.get()));
+        if (d->elec >= 0) {
+            cudaResourceDesc r{};
+            r.resType = cudaResourceTypeLinear;
+            r.res.linear.devPtr = d->d_eps;
+            r.res.linear.desc = cudaCreateChannelDesc<float2>();
+            r.res.linear.sizeInBytes = AG_NDIEL * sizeof(float2);
+            cudaTextureDesc td{};
+            td.readMode = cudaReadModeElementType;
+            DF_CK(cudaCreateTextureObject(&d->eps_tex, &r, &td, nullptr));
+        }
         A.row_v = (const float *)d->d_vdw;
         A.row_d = A.row_v + n_rows * A.row_stride;
     }
@@ -543,7 +560,11 @@ ag_status ag_diff_forward(ag_diff *d, int32_t keep_closest_h, void *device_out)
         }
     }
     DF_CK(cudaEventRecord(d->ev[0], s));
-    if (d->elec >= 0) DF_CK(launch_emap_lin(d->fp64, A, d->d_eps, out + d->esz * d->P * d->elec, s));
+    if (d->elec >= 0) {
+        unsigned char *em = out + d->esz * d->P * d->elec;
+        if (d->fp64) DF_CK(launch_emap_lin(A, d->d_eps, (double *)em, s));
+        else DF_CK(launch_elin(A, d->d_eps, d->eps_tex, (float *)em, d->d_epart, s));
+    }
     if (d->fp64) DF_CK(launch_near_lin(A, d->d_vdw, d->d_sol, (double *)out, d->d_ch, d->d_mmarg, s));
     else DF_CK(launch_rows(A, d->d_sol, (float *)out, d->d_ch, d->d_mmarg, s));
     if (d->floating || d->constriction)
@@ -620,7 +641,11 @@ ag_status ag_diff_backward(ag_diff *d, const void *grad_maps, int32_t grad_on_de
     g.rv2 = d->d_grad + 7 * N;
     DF_CK(cudaMemsetAsync(d->d_grad, 0, 10 * N * K * sizeof(double), s));
     DF_CK(cudaEventRecord(d->ev[2], s));
-    if (d->elec >= 0) DF_CK(launch_emap_lin_adj(d->fp64, d->args, d->d_eps, gm + d->esz * d->P * d->elec, g, s));
+    if (d->elec >= 0) {
+        const unsigned char *ge = gm + d->esz * d->P * d->elec;
+        if (d->fp64) DF_CK(launch_emap_lin_adj(d->args, d->d_eps, (const double *)ge, g, s));
+        else DF_CK(launch_elin_adj(d->args, d->d_eps, d->eps_tex, (const float *)ge, g, s));
+    }
     if (d->fp64)
         DF_CK(launch_near_lin_adj(d->args, d->d_vdw, d->d_sol, (const double *)gm, d->d_ch, d->d_mmarg, g, s));
     else

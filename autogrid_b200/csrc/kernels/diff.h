@@ -139,9 +139,17 @@ cudaError_t launch_bond_vectors(int K, int N, const int *topo, const double *x, 
 cudaError_t launch_bond_vectors_adj(int K, int N, const int *topo, const double *x, const double *y, const double *z,
                                     const double *grad, double *gx, cudaStream_t s);
 cudaError_t launch_cell_lists(const DiffArgs &a, int *cell_of, int *count, cudaStream_t s);
-cudaError_t launch_emap_lin(bool fp64, const DiffArgs &a, const void *eps, void *emap, cudaStream_t s);
-cudaError_t launch_emap_lin_adj(bool fp64, const DiffArgs &a, const void *eps, const void *g_e, DiffGrads g,
-                                cudaStream_t s);
+// e map: the FP64 twin (kernels/diff_emap.cu) and the FP32 kernels
+// (kernels/diff_emap_rows.cu; partial: elin_chunks(a) * P * n_conf floats when
+// there are several chunks).
+cudaError_t launch_emap_lin(const DiffArgs &a, const void *eps, double *emap, cudaStream_t s);
+cudaError_t launch_emap_lin_adj(const DiffArgs &a, const void *eps, const double *g_e, DiffGrads g, cudaStream_t s);
+int elin_chunks(const DiffArgs &a);
+cudaError_t prepare_elin();  // shared-memory limits on the current device
+cudaError_t launch_elin(const DiffArgs &a, const void *eps, cudaTextureObject_t tex, float *emap, float *partial,
+                        cudaStream_t s);
+cudaError_t launch_elin_adj(const DiffArgs &a, const void *eps, cudaTextureObject_t tex, const float *g_e, DiffGrads g,
+                            cudaStream_t s);
 // The FP64 twin (kernels/diff_near.cu) and the FP32 kernels (kernels/diff_rows.cu).
 cudaError_t launch_near_lin(const DiffArgs &a, const void *vdw, const void *sol, double *maps, const int *ch, int *mmarg,
                             cudaStream_t s);
