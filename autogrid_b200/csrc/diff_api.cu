@@ -474,7 +474,13 @@ ag_status ag_diff_create_batch(ag_context *ctx, const ag_problem *p, const ag_op
         });
         std::vector<R2<float>> sol, eps;
         build_tables(p, sol, eps);
-        DF_CK(put(&d->d_vdw, rows, d.get())); DF_CK(put(&d->d_sol, sol, d.get())); DF_CK(put(&d->d_eps, eps, d.get()));
+        DF_CK(put(&d->d_vdw, rows, d.get())); DF_CK(put(&d->d_sol, sol, d.get()));
+        // the dielectric table starts where a texture can (512 bytes)
+        constexpr size_t kAlign = 512;
+        unsigned char *room = nullptr;
+        DF_CK(d->alloc(&room, eps.size() * sizeof(eps[0]) + kAlign));
+        d->d_eps = (void *)(((size_t)room + kAlign - 1) / kAlign * kAlign);
+        DF_CK(cudaMemcpy(d->d_eps, eps.data(), eps.size() * sizeof(eps[0]), cudaMemcpyHostToDevice));
         if (d->elec >= 0) {
             cudaResourceDesc r{};
             r.resType = cudaResourceTypeLinear;
