@@ -467,10 +467,14 @@ ag_status ag_diff_create_batch(ag_context *ctx, const ag_problem *p, const ag_op
         build_tables(p, sol, eps);
         DF_CK(put(&d->d_vdw, vdw, d.get())); DF_CK(put(&d->d_sol, sol, d.get())); DF_CK(put(&d->d_eps, eps, d.get()));
     } else {
-        std::vector<float> rows(2 * n_rows * A.row_stride, 0.f);  // values, then steps
+        // values, then steps; a type's last value row is there twice
+        const size_t n32 = n_rows / AG_NEINT * DF_ROWS;
+        std::vector<float> rows(2 * n32 * A.row_stride, 0.f);
         each_vdw(p, A, [&](size_t row, int s, double v, double dv) {
-            rows[row * A.row_stride + s] = (float)v;
-            rows[(n_rows + row) * A.row_stride + s] = (float)dv;
+            const size_t t = row / AG_NEINT, b = row % AG_NEINT, o = (t * DF_ROWS + b) * A.row_stride + s;
+            rows[o] = (float)v;
+            rows[n32 * A.row_stride + o] = (float)dv;
+            if (b == AG_NEINT - 1) rows[o + A.row_stride] = (float)v;
         });
         std::vector<R2<float>> sol, eps;
         build_tables(p, sol, eps);
@@ -492,7 +496,7 @@ ag_status ag_diff_create_batch(ag_context *ctx, const ag_problem *p, const ag_op
             DF_CK(cudaCreateTextureObject(&d->eps_tex, &r, &td, nullptr));
         }
         A.row_v = (const float *)d->d_vdw;
-        A.row_d = A.row_v + n_rows * A.row_stride;
+        A.row_d = A.row_v + n32 * A.row_stride;
     }
     A.x = d->d_x; A.y = d->d_y; A.z = d->d_z; A.q = d->d_q; A.vol = d->d_vol; A.solpar = d->d_solpar;
     A.rv = d->d_rv; A.rv2 = d->d_rv2; A.meta = d->d_meta; A.h_index = d->d_h;

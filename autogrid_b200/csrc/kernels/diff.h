@@ -32,6 +32,7 @@ constexpr int DF_MAXMM = 8;   // slots that keep an H-bond min/max
 constexpr int DF_BRICK_X = 8, DF_BRICK_Y = 8, DF_BRICK_Z = 4;
 constexpr int DF_THREADS = DF_BRICK_X * DF_BRICK_Y * DF_BRICK_Z;
 constexpr int DF_STAGE = 256;       // candidate atoms staged in shared memory at once
+constexpr int DF_ROWS = AG_NEINT + 1;  // FP32 table rows of a type: the bins, the last one again
 constexpr double DF_RADIUS = 8.05;  // cell acceptance radius (A), > the 8 A cutoff
 
 // What a (slot, receptor class) pair adds, after main.cpp:3290-3379.
@@ -82,8 +83,8 @@ struct DiffArgs {
     int slot_desolv[DF_MAXS];    // 1: receives a desolvation term
     double slot_sp[DF_MAXS], slot_vp[DF_MAXS];
     uint8_t act[DF_MAXS][16];    // [slot][hbond + 8 * disorder]
-    // FP32 kernels (diff_rows.cu): value and step rows [type][bin][row_stride],
-    // row_stride a multiple of 8; the actions of a class, 4 bits per slot; the
+    // FP32 kernels (diff_rows.cu): value and step rows
+    // [type][DF_ROWS][row_stride], row_stride a multiple of 8; the actions of a class, 4 bits per slot; the
     // classes whose every slot is plain; slots [0, n_hb) hold every slot with
     // an H-bond action
     const float *row_v, *row_d;

@@ -11,22 +11,26 @@
 //                Hramp gradient on the closest hydrogen is added per point.
 //
 // Table rows.  Row (type, bin) of row_v and row_d holds the value and the step
-// to the next bin of every slot, 8 (or 16) floats, one 32-byte load each.  For
-// most receptor classes every slot is the plain T = v + f d, and the row is
-// 4 (8) packed multiply-adds; only classes with an H-bond action walk the
-// slots one by one.  The desolvation terms of all slots factor into two sums
+// to the next bin of every slot, 8 (or 16) floats, one 32-byte load each.  The
+// forward reads the value rows of the bin and the next one and subtracts (the
+// steps exactly, as the tables are FP32), which keeps its tables at half the
+// size in L1; candidates are staged in the order of their types for the same
+// reason.  For most receptor classes every slot is the plain T = v + f d, and
+// the row is 4 (8) packed multiply-adds; only classes with an H-bond action
+// walk the slots one by one.  The desolvation terms of all slots factor into two sums
 // per point, D1 = sum w sol vol and D2 = sum w sol (solpar + qasp |q|):
 // slot s ends with sp_s D1 + vp_s D2.  In the adjoint a plain pair below the
 // last bin (w = 1, dw = 0) needs the steps alone: half the bytes.
 //
-// What bounds it: the forward, the L1 data path of the row gathers (86% busy;
-// a 32-byte gather takes one wavefront per lane, 20.6 per request, where two
-// 16-byte ones took 30.8); the adjoint, issue (64%) and that path (67%).  Eight
-// conformers of 8,000 atoms, 101^3 points, 8 Vina maps: forward 3.6 ms,
-// adjoint 2.9 ms; kernels that walked the slots of every pair one by one took
-// 8.6 and 12.8 ms (295 and 475 instructions per warp and candidate, now 61 and
-// 113).  4,000 atoms, 61^3 points, 8 AD4 maps: 0.39 -> 0.17 ms and 0.75 ->
-// 0.36 ms.
+// What bounds it: the forward, the L1 data path of the row gathers (85% busy, at
+// one wavefront per lane for a 32-byte gather that hits L1, two for a miss);
+// the adjoint, issue (64%) and that path (69%).  Eight conformers of 8,000
+// atoms, 101^3 points, 8 Vina maps: forward 3.1 ms, adjoint 3.0 ms; kernels that
+// walked the slots of every pair one by one took 8.6 and 12.8 ms (295 and 475
+// instructions per warp and candidate, now 65 and 101).  Rows in the order of
+// the candidates' cells instead of their types, and step rows in the forward,
+// hit L1 for 58% instead of 89%: forward 3.6 ms.  4,000 atoms, 61^3 points,
+// 8 AD4 maps: 0.39 -> 0.17 ms and 0.75 -> 0.33 ms.
 #include "diff_pair.cuh"
 
 #include "diff_brick.cuh"
@@ -60,7 +64,10 @@ template <bool ANG, bool SOL> struct RowsSmem {
     float4 aux[SOL || ANG ? DF_STAGE : 1];      // vol, solpar + qasp |q|, qasp sgn(q), -
     int idx[DF_STAGE];
     float4 rv[ANG ? DF_STAGE : 1], rv2[ANG ? DF_STAGE : 1];
-    unsigned short wl[DF_WARPS][DF_STAGE];      // per warp: staged slots near its points
+    union {
+        unsigned short wl[DF_WARPS][DF_STAGE];  // per warp: staged slots near its points
+        int tcnt[DF_STAGE / 32][32];            // staging by receptor type: per 32-candidate slice and type
+    };
     float wbox[DF_WARPS][6];                    // per warp: its points' box (lo xyz, hi xyz), A
     float2 sol[SOL ? AG_NEINT : 1];
     unsigned long long act[ANG ? 16 : 1];
@@ -97,25 +104,60 @@ __device__ __forceinline__ void rows_box(const Brick &bk, float px, float py, fl
     __syncwarp();
 }
 
-// Stage candidates [c0, c0 + DF_STAGE) of the brick.
+// Stage candidates [c0, c0 + DF_STAGE) of the brick, ordered by receptor type
+// by a stable counting sort (cell order within a type), so that the warps walk
+// the table of one type at a time.  Slice k (one warp's candidates) is ranked
+// by its warp; tcnt[k][t] holds the slice's count of type t, then the slot of
+// its first such candidate.  All threads call it; it ends with a barrier.
 template <bool ANG, bool SOL>
 __device__ __forceinline__ void rows_stage(const DiffArgs &a, const ConfView &v, RowsSmem<ANG, SOL> &sm, int c0)
 {
     static_assert(DF_STAGE == DF_THREADS, "one candidate per thread");
-    const int t = threadIdx.x;
-    if (c0 + t >= sm.sg.total) return;
-    const int ia = brick_atom(v, sm.sg, c0 + t);
-    sm.pos[t] = make_float4((float)v.x[ia], (float)v.y[ia], (float)v.z[ia], __int_as_float(a.meta[ia]));
-    sm.idx[t] = ia;
-    if (SOL) {
-        const float q = (float)v.q[ia], qasp = (float)a.solpar_q;
-        sm.aux[t] = make_float4((float)a.vol[ia], (float)a.solpar[ia] + qasp * fabsf(q),
-                                q > 0.f ? qasp : (q < 0.f ? -qasp : 0.f), 0.f);
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    const bool in = c0 + t < sm.sg.total;
+    sm.tcnt[w][lane] = 0;
+    const int ia = in ? brick_atom(v, sm.sg, c0 + t) : 0;
+    const int meta = in ? a.meta[ia] : 0, type = in ? meta & DM_TYPE_MASK : 32;  // 32: past the chunk
+    const unsigned same = __match_any_sync(0xffffffffu, type);
+    const int rank = __popc(same & ((1u << lane) - 1u));
+    if (in && rank == 0) sm.tcnt[w][type] = __popc(same);
+    __syncthreads();
+    if (w == 0) {  // lane: a type's slots, slices in order, after every lower type
+        int cnt[DF_WARPS], run = 0;
+#pragma unroll
+        for (int k = 0; k < DF_WARPS; k++) {
+            cnt[k] = sm.tcnt[k][lane];
+            run += cnt[k];
+        }
+        int first = run;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, first, o);
+            if (lane >= o) first += u;
+        }
+        first -= run;
+#pragma unroll
+        for (int k = 0; k < DF_WARPS; k++) {
+            sm.tcnt[k][lane] = first;
+            first += cnt[k];
+        }
     }
-    if (ANG) {
-        sm.rv[t] = make_float4((float)v.rv[3 * ia], (float)v.rv[3 * ia + 1], (float)v.rv[3 * ia + 2], 0.f);
-        sm.rv2[t] = make_float4((float)v.rv2[3 * ia], (float)v.rv2[3 * ia + 1], (float)v.rv2[3 * ia + 2], 0.f);
+    __syncthreads();
+    if (in) {
+        const int j = sm.tcnt[w][type] + rank;
+        sm.pos[j] = make_float4((float)v.x[ia], (float)v.y[ia], (float)v.z[ia], __int_as_float(meta));
+        sm.idx[j] = ia;
+        if (SOL) {
+            const float q = (float)v.q[ia], qasp = (float)a.solpar_q;
+            sm.aux[j] = make_float4((float)a.vol[ia], (float)a.solpar[ia] + qasp * fabsf(q),
+                                    q > 0.f ? qasp : (q < 0.f ? -qasp : 0.f), 0.f);
+        }
+        if (ANG) {
+            sm.rv[j] = make_float4((float)v.rv[3 * ia], (float)v.rv[3 * ia + 1], (float)v.rv[3 * ia + 2], 0.f);
+            sm.rv2[j] = make_float4((float)v.rv2[3 * ia], (float)v.rv2[3 * ia + 1], (float)v.rv2[3 * ia + 2], 0.f);
+        }
     }
+    __syncthreads();
 }
 
 // Slots j < n of the staged chunk whose atom lies within the cutoff + 0.01 A
@@ -145,7 +187,7 @@ template <class SM> __device__ __forceinline__ int rows_candidates(SM &sm, int n
     return cnt;
 }
 
-// Geometry of one pair; false beyond 8 A.  The same operations as dfm::geom.
+// Geometry of one pair; false beyond 8 A.
 struct RowGeom {
     float d[3], inv, x, fx, w;
     int b;
@@ -157,10 +199,15 @@ __device__ __forceinline__ bool rows_geom(const float4 &A, float px, float py, f
     g.d[2] = A.z - pz;
     // r picks the table bin, where the slopes jump: its rounding is pinned, so
     // that forward and adjoint (and later builds) take the same bins
-    const float r2 = __fmaf_rn(g.d[2], g.d[2], __fmaf_rn(g.d[1], g.d[1], __fmul_rn(g.d[0], g.d[0])));
+    float r2 = __fmaf_rn(g.d[2], g.d[2], __fmaf_rn(g.d[1], g.d[1], __fmul_rn(g.d[0], g.d[0])));
     if (r2 > (float)(AG_NBC * AG_NBC)) return false;
-    float r;
-    dist_inv(r2, r, g.inv);
+    // r = sqrt(r2), at least 1e-6 A, by Markstein's correction of r2 * (1/sqrt(r2)),
+    // which shares the approximation with 1/r; correctly rounded for every
+    // float in [1e-13, 65] (all of them compared with sqrtf)
+    r2 = fmaxf(r2, 1.0e-12f);
+    g.inv = rsqrt_approx(r2);
+    const float r1 = __fmul_rn(r2, g.inv);
+    const float r = __fmaf_rn(__fmaf_rn(-r1, r1, r2), 0.5f * g.inv, r1);
     g.x = r * (float)AG_A_DIV;
     g.b = min((int)g.x, AG_NEINT - 1);
     g.fx = g.x - (float)g.b;
@@ -179,7 +226,7 @@ __device__ __forceinline__ float th_row(const DiffArgs &a, int s, float x, float
     if (a.hydrogen_type < 0 || a.hydrogen_type >= a.n_rec_types) return 0.f;
     const float xh = x - (float)(1.10 * AG_A_DIV);
     const int bh = xh <= 0.f ? 0 : min((int)xh, AG_NEINT - 1);
-    const size_t o = ((size_t)a.hydrogen_type * AG_NEINT + bh) * a.row_stride + s;
+    const size_t o = ((size_t)a.hydrogen_type * DF_ROWS + bh) * a.row_stride + s;
     const float v = __ldg(a.row_v + o);
     if (xh <= 0.f) return v;
     dth = __ldg(a.row_d + o);
@@ -221,7 +268,6 @@ k_rows(DiffArgs a, const float2 *__restrict__ sol, float *__restrict__ maps, con
     for (int c0 = 0; c0 < sm.sg.total; c0 += DF_STAGE) {
         if (c0) __syncthreads();
         rows_stage(a, v, sm, c0);
-        __syncthreads();
         const int cnt = rows_candidates(sm, min(DF_STAGE, sm.sg.total - c0));
         if (!bk.valid) continue;
         for (int k = 0; k < cnt; k++) {
@@ -230,13 +276,13 @@ k_rows(DiffArgs a, const float2 *__restrict__ sol, float *__restrict__ maps, con
             RowGeom g;
             if (!rows_geom(A, px, py, pz, g)) continue;
             const int meta = __float_as_int(A.w);
-            const unsigned ro = (unsigned)((meta & DM_TYPE_MASK) * AG_NEINT + g.b) * (unsigned)a.row_stride;
+            const unsigned ro = (unsigned)((meta & DM_TYPE_MASK) * DF_ROWS + g.b) * (unsigned)a.row_stride;
             Row8 rv8[NB], rd8[NB];
 #pragma unroll
             for (int k8 = 0; k8 < NB; k8++)
                 if (8 * k8 < a.n_slots) {
                     rv8[k8] = load_row8(a.row_v + ro + 8 * k8);
-                    rd8[k8] = load_row8(a.row_d + ro + 8 * k8);
+                    rd8[k8] = load_row8(a.row_v + ro + a.row_stride + 8 * k8);  // the next bin's values
                 }
             if (SOL) {
                 const float2 t = sm.sol[g.b];
@@ -245,6 +291,12 @@ k_rows(DiffArgs a, const float2 *__restrict__ sol, float *__restrict__ maps, con
                 D1 = fmaf(ws, x.x, D1);
                 D2 = fmaf(ws, x.y, D2);
             }
+#pragma unroll
+            for (int k8 = 0; k8 < NB; k8++)
+                if (8 * k8 < a.n_slots)
+#pragma unroll
+                    for (int i = 0; i < 4; i++)
+                        rd8[k8].p[i] = __fadd2_rn(rd8[k8].p[i], make_float2(-rv8[k8].p[i].x, -rv8[k8].p[i].y));
             const float2 f2 = both(g.fx), w2 = both(g.w);
             const int cls = ANG ? ((meta >> DM_HB_SHIFT) & 7) + ((meta & DM_DIS) ? 8 : 0) : 0;
             if (!ANG || ((a.cls_plain >> cls) & 1u)) {
@@ -313,6 +365,51 @@ k_rows(DiffArgs a, const float2 *__restrict__ sol, float *__restrict__ maps, con
     }
 }
 
+// Adjoint of one in-range pair of a class whose slots are all plain:
+// dL/d(atom position) and, with desolvation, dL/dq.
+template <int NB, bool SOL>
+__device__ __forceinline__ void plain_adjoint(const DiffArgs &a, const RowGeom &g, unsigned ro, const float2 *sol,
+                                              const float4 *aux, const float2 (&gs)[4 * NB], float gD1, float gD2,
+                                              float *out)
+{
+    const float dw = (float)AG_NEINT - g.x < 1.f ? -1.f : 0.f;
+    float G_x = 0.f;
+    Row8 rd8[NB];
+#pragma unroll
+    for (int k8 = 0; k8 < NB; k8++)
+        if (8 * k8 < a.n_slots) rd8[k8] = load_row8(a.row_d + ro + 8 * k8);
+    if (SOL) {
+        const float2 t = sol[g.b];
+        const float4 x = *aux;
+        const float so = fmaf(g.fx, t.y, t.x);
+        G_x = fmaf(dw, so, g.w * t.y) * fmaf(x.y, gD2, x.x * gD1);
+        out[3] = g.w * so * x.z * gD2;
+    }
+    float2 S = both(0.f);
+#pragma unroll
+    for (int k8 = 0; k8 < NB; k8++)
+        if (8 * k8 < a.n_slots)
+#pragma unroll
+            for (int i = 0; i < 4; i++) S = __ffma2_rn(gs[4 * k8 + i], rd8[k8].p[i], S);
+    G_x = fmaf(g.w, S.x + S.y, G_x);
+    if (dw != 0.f) {  // the last bin: the switch's own slope
+        const float2 f2 = both(g.fx);
+        S = both(0.f);
+#pragma unroll
+        for (int k8 = 0; k8 < NB; k8++)
+            if (8 * k8 < a.n_slots) {
+                const Row8 r = load_row8(a.row_v + ro + 8 * k8);
+#pragma unroll
+                for (int i = 0; i < 4; i++) S = __ffma2_rn(gs[4 * k8 + i], __ffma2_rn(f2, rd8[k8].p[i], r.p[i]), S);
+            }
+        G_x -= S.x + S.y;
+    }
+    const float gx = G_x * (float)AG_A_DIV * g.inv;
+    out[0] = gx * g.d[0];
+    out[1] = gx * g.d[1];
+    out[2] = gx * g.d[2];
+}
+
 template <int MS, int MM, int MINB, bool ANG, bool SOL>
 __global__ void __launch_bounds__(DF_THREADS, MINB)
 k_rows_adj(DiffArgs a, const float2 *__restrict__ sol, const float *__restrict__ g_maps, const int *__restrict__ chs,
@@ -369,8 +466,30 @@ k_rows_adj(DiffArgs a, const float2 *__restrict__ sol, const float *__restrict__
     for (int c0 = 0; c0 < sm.sg.total; c0 += DF_STAGE) {
         if (c0) __syncthreads();
         rows_stage(a, v, sm, c0);
-        __syncthreads();
         const int cnt = rows_candidates(sm, min(DF_STAGE, sm.sg.total - c0));
+        if (!ANG) {
+            // two candidates at a time: their chains overlap, and one pass of
+            // shuffles sums both
+            for (int k = 0; k < cnt; k += 2) {
+                float out[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                for (int u = 0; u < 2; u++) {
+                    const int j = wl[min(k + u, cnt - 1)];
+                    const float4 A = sm.pos[j];
+                    RowGeom g;
+                    if (!rows_geom(A, px, py, pz, g) || !bk.valid || k + u >= cnt) continue;
+                    const unsigned ro = (unsigned)((__float_as_int(A.w) & DM_TYPE_MASK) * DF_ROWS + g.b) * (unsigned)a.row_stride;
+                    plain_adjoint<NB, SOL>(a, g, ro, sm.sol, sm.aux + (SOL ? j : 0), gs, gD1, gD2, out + 4 * u);
+                }
+                const float sum = warp_sums(out, lane);
+                const int n = (lane >> 2) & 3, u = lane >> 4;
+                if ((lane & 3) == 0 && (SOL || n < 3) && k + u < cnt && sum != 0.f) {
+                    const long long ia = sm.idx[wl[k + u]];
+                    atomicAdd(n < 3 ? gr.xyz + 3 * ia + n : gr.q + ia, (double)sum);
+                }
+            }
+            continue;
+        }
         for (int k = 0; k < cnt; k++) {
             const int j = wl[k];
             const float4 A = sm.pos[j];
@@ -382,52 +501,28 @@ k_rows_adj(DiffArgs a, const float2 *__restrict__ sol, const float *__restrict__
             const bool plain = !ANG || ((a.cls_plain >> cls) & 1u);
             float out[4] = {0.f, 0.f, 0.f, 0.f};
             float g_rv[3] = {0.f, 0.f, 0.f}, g_rv2[3] = {0.f, 0.f, 0.f};
+            const unsigned ro = (unsigned)((meta & DM_TYPE_MASK) * DF_ROWS + g.b) * (unsigned)a.row_stride;
             if (in) {
-                const unsigned ro = (unsigned)((meta & DM_TYPE_MASK) * AG_NEINT + g.b) * (unsigned)a.row_stride;
-                const float dw = (float)AG_NEINT - g.x < 1.f ? -1.f : 0.f;
-                float G_x = 0.f;
-                Row8 rd8[NB];
-#pragma unroll
-                for (int k8 = 0; k8 < NB; k8++)
-                    if (8 * k8 < a.n_slots) rd8[k8] = load_row8(a.row_d + ro + 8 * k8);
-                if (SOL) {
-                    const float2 t = sm.sol[g.b];
-                    const float4 x = sm.aux[j];
-                    const float so = fmaf(g.fx, t.y, t.x);
-                    G_x = fmaf(dw, so, g.w * t.y) * fmaf(x.y, gD2, x.x * gD1);
-                    out[3] = g.w * so * x.z * gD2;
-                }
-                const float dn[3] = {g.d[0] * g.inv, g.d[1] * g.inv, g.d[2] * g.inv};
                 if (plain) {
-                    float2 S = both(0.f);
-#pragma unroll
-                    for (int k8 = 0; k8 < NB; k8++)
-                        if (8 * k8 < a.n_slots)
-#pragma unroll
-                            for (int i = 0; i < 4; i++) S = __ffma2_rn(gs[4 * k8 + i], rd8[k8].p[i], S);
-                    G_x = fmaf(g.w, S.x + S.y, G_x);
-                    if (dw != 0.f) {  // the last bin: the switch's own slope
-                        const float2 f2 = both(g.fx);
-                        S = both(0.f);
-#pragma unroll
-                        for (int k8 = 0; k8 < NB; k8++)
-                            if (8 * k8 < a.n_slots) {
-                                const Row8 r = load_row8(a.row_v + ro + 8 * k8);
-#pragma unroll
-                                for (int i = 0; i < 4; i++)
-                                    S = __ffma2_rn(gs[4 * k8 + i], __ffma2_rn(f2, rd8[k8].p[i], r.p[i]), S);
-                            }
-                        G_x -= S.x + S.y;
-                    }
-                    const float gx = G_x * (float)AG_A_DIV;
-                    out[0] = gx * dn[0];
-                    out[1] = gx * dn[1];
-                    out[2] = gx * dn[2];
+                    plain_adjoint<NB, SOL>(a, g, ro, sm.sol, sm.aux + (SOL ? j : 0), gs, gD1, gD2, out);
                 } else {
-                    Row8 rv8[NB];
+                    const float dw = (float)AG_NEINT - g.x < 1.f ? -1.f : 0.f;
+                    const float dn[3] = {g.d[0] * g.inv, g.d[1] * g.inv, g.d[2] * g.inv};
+                    float G_x = 0.f;
+                    Row8 rd8[NB], rv8[NB];
 #pragma unroll
                     for (int k8 = 0; k8 < NB; k8++)
-                        if (8 * k8 < a.n_slots) rv8[k8] = load_row8(a.row_v + ro + 8 * k8);
+                        if (8 * k8 < a.n_slots) {
+                            rd8[k8] = load_row8(a.row_d + ro + 8 * k8);
+                            rv8[k8] = load_row8(a.row_v + ro + 8 * k8);
+                        }
+                    if (SOL) {
+                        const float2 t = sm.sol[g.b];
+                        const float4 x = sm.aux[j];
+                        const float so = fmaf(g.fx, t.y, t.x);
+                        G_x = fmaf(dw, so, g.w * t.y) * fmaf(x.y, gD2, x.x * gD1);
+                        out[3] = g.w * so * x.z * gD2;
+                    }
                     const float4 r1 = sm.rv[j], r2 = sm.rv2[j];
                     const float rv[3] = {r1.x, r1.y, r1.z}, rv2[3] = {r2.x, r2.y, r2.z};
                     const int hb = cls & 7;
@@ -502,15 +597,15 @@ k_rows_adj(DiffArgs a, const float2 *__restrict__ sol, const float *__restrict__
 // The instantiation of a map set: 8 or 16 slots; no, at most 2 or at most 8
 // min/max slots; directional factors or not; desolvation terms or not.
 // <MS, MM, blocks per SM>: the Vina maps measured the same with 3 and 4 blocks
-// and 3-5% slower with 5 and 6 (the registers spill); the 8-slot AD4 sets the
-// same with 2 and 3 and 1% slower with 4.
-#define ROWS_LAUNCH(KERNEL, ...)                                                                          \
+// and 3-5% slower with 5 and 6 (the registers spill); the 8-slot AD4 forward
+// the same with 2 and 3, its adjoint 10% faster with 2 (it spills with 3).
+#define ROWS_LAUNCH(KERNEL, AD4, ...)                                                                          \
     do {                                                                                                  \
         const bool small = a.n_slots <= 8;                                                                \
         if (!a.need_ang && small && !a.need_sol) KERNEL<8, 0, 4, false, false><<<brick_grid(a), DF_THREADS, 0, s>>>(__VA_ARGS__);  \
         else if (!a.need_ang && small) KERNEL<8, 0, 4, false, true><<<brick_grid(a), DF_THREADS, 0, s>>>(__VA_ARGS__);             \
         else if (!a.need_ang) KERNEL<16, 0, 3, false, true><<<brick_grid(a), DF_THREADS, 0, s>>>(__VA_ARGS__);                     \
-        else if (small && a.n_mm <= 2) KERNEL<8, 2, 3, true, true><<<brick_grid(a), DF_THREADS, 0, s>>>(__VA_ARGS__);              \
+        else if (small && a.n_mm <= 2) KERNEL<8, 2, AD4, true, true><<<brick_grid(a), DF_THREADS, 0, s>>>(__VA_ARGS__);              \
         else if (a.n_mm <= 2) KERNEL<16, 2, 2, true, true><<<brick_grid(a), DF_THREADS, 0, s>>>(__VA_ARGS__);                      \
         else KERNEL<16, DF_MAXMM, 2, true, true><<<brick_grid(a), DF_THREADS, 0, s>>>(__VA_ARGS__);                                \
     } while (0)
@@ -520,7 +615,7 @@ k_rows_adj(DiffArgs a, const float2 *__restrict__ sol, const float *__restrict__
 cudaError_t launch_rows(const DiffArgs &a, const void *sol, float *maps, const int *ch, int *mmarg, cudaStream_t s)
 {
     if (a.P == 0 || a.n_slots == 0) return cudaSuccess;
-    ROWS_LAUNCH(k_rows, a, (const float2 *)sol, maps, ch, mmarg);
+    ROWS_LAUNCH(k_rows, 3, a, (const float2 *)sol, maps, ch, mmarg);
     return cudaGetLastError();
 }
 
@@ -528,7 +623,7 @@ cudaError_t launch_rows_adj(const DiffArgs &a, const void *sol, const float *g_m
                             DiffGrads g, cudaStream_t s)
 {
     if (a.P == 0 || a.n_slots == 0) return cudaSuccess;
-    ROWS_LAUNCH(k_rows_adj, a, (const float2 *)sol, g_maps, ch, mmarg, g);
+    ROWS_LAUNCH(k_rows_adj, 2, a, (const float2 *)sol, g_maps, ch, mmarg, g);
     return cudaGetLastError();
 }
 
