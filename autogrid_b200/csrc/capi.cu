@@ -243,6 +243,31 @@ struct ag_context {
     size_t h_text_cap = 0;
     cudaEvent_t tev[4] = {nullptr, nullptr, nullptr, nullptr};  // measure and write passes
     BufferSet table_bufs;  // ag_tables_build
+    // pinned host image of a one-shot call's inputs (Stage)
+    char *h_stage = nullptr;
+    size_t h_stage_cap = 0;
+    // The image with room for `bytes`, null where no memory can be pinned.
+    // s: the stream of the previous call's copies; they are done when that
+    // call has returned, unless it failed on its way.
+    cudaError_t stage(size_t bytes, cudaStream_t s, char **out)
+    {
+        *out = nullptr;
+        const cudaError_t e = cudaStreamSynchronize(s);
+        if (e != cudaSuccess) return e;
+        if (bytes > h_stage_cap) {
+            if (h_stage) cudaFreeHost(h_stage);
+            h_stage = nullptr;
+            h_stage_cap = 0;
+            if (cudaHostAlloc((void **)&h_stage, bytes, cudaHostAllocDefault) != cudaSuccess) {
+                cudaGetLastError();
+                h_stage = nullptr;
+                return cudaSuccess;
+            }
+            h_stage_cap = bytes;
+        }
+        *out = h_stage;
+        return cudaSuccess;
+    }
     // the last run, whose statistics ag_context_stats() settles
     bool pending = false, had_far = false;
     int last_launches = 0;
@@ -380,18 +405,59 @@ bool is_device_memory(const void *ptr)
 }
 
 template <class T>
-cudaError_t upload(BufferSet *b, const char *name, const T *src, size_t n, T **dst, cudaStream_t s, size_t *acc)
+cudaError_t upload(BufferSet *b, const char *name, const T *src, size_t n, T **dst, cudaStream_t s)
 {
     void *d = nullptr;
     cudaError_t e = b->ensure(name, n * sizeof(T), &d);
     if (e != cudaSuccess) return e;
     *dst = (T *)d;
-    if (n) {
-        e = cudaMemcpyAsync(d, src, n * sizeof(T), cudaMemcpyHostToDevice, s);
-        if (acc) *acc += n * sizeof(T);
-    }
-    return e;
+    return n ? cudaMemcpyAsync(d, src, n * sizeof(T), cudaMemcpyHostToDevice, s) : cudaSuccess;
 }
+
+// The host image of several input arrays of a plan, sent to the device in one
+// copy: a copy for each array, 25 of them, cost 90 us of host time in a
+// 41^3-point one-shot call of 0.47 ms.  The image lies in `pinned`
+// (room(bytes, arrays) of it), or in memory of its own.
+struct Stage {
+    static constexpr size_t kAlign = 256;
+    std::unique_ptr<char[]> own;
+    char *buf;
+    size_t cap, used = 0;
+    std::vector<std::pair<size_t, void **>> dst;
+    static size_t room(size_t bytes, int arrays) { return (bytes + kAlign * (size_t)arrays + kAlign - 1) / kAlign * kAlign; }
+    Stage(size_t bytes, int arrays, char *pinned) : buf(pinned), cap(room(bytes, arrays))
+    {
+        if (!pinned) {
+            own.reset(new char[cap]);
+            buf = own.get();
+        }
+    }
+    template <class T>
+    T *make(size_t n, T **d)
+    {
+        T *r = (T *)(buf + used);
+        dst.emplace_back(used, (void **)d);
+        used += (std::max<size_t>(n, 1) * sizeof(T) + kAlign - 1) / kAlign * kAlign;
+        return used <= cap ? r : nullptr;
+    }
+    template <class T>
+    bool add(const T *src, size_t n, T **d)
+    {
+        T *r = make(n, d);
+        if (r && n) std::memcpy(r, src, n * sizeof(T));
+        return r != nullptr;
+    }
+    cudaError_t send(BufferSet *b, const char *name, cudaStream_t s, size_t *acc)
+    {
+        if (used > cap) return cudaErrorInvalidValue;
+        void *d = nullptr;
+        cudaError_t e = b->ensure(name, used, &d);
+        if (e != cudaSuccess) return e;
+        for (auto &x : dst) *x.second = (char *)d + x.first;
+        *acc += used;
+        return used ? cudaMemcpyAsync(d, buf, used, cudaMemcpyHostToDevice, s) : cudaSuccess;
+    }
+};
 
 // Error bounds of the canonical FP32 distances for a grid spacing (in bins):
 // the far kernel's bin-guard multipliers and the near kernel's guard, from the
@@ -410,6 +476,23 @@ void far_guard(double spacing_adiv, float *lo, float *hi, float *near)
     const double p_max = std::sqrt(px * px + 2 * pyz * pyz);
     far_edge_multipliers(p_max, exact, 2.5, lo, hi);
     *near = near_edge_guard(p_max, exact, 2.5);
+}
+
+// Cells per axis of the cell list over the grid box grown by the near radius.
+void cell_grid(const ag_problem *p, int nc[3], double lo[3], double hi[3])
+{
+    for (int i = 0; i < 3; i++) {
+        lo[i] = (double)(-p->ne[i]) * p->spacing - AGB_NEAR_RADIUS;
+        hi[i] = (double)(p->n1[i] - 1 - p->ne[i]) * p->spacing + AGB_NEAR_RADIUS;
+        nc[i] = std::max(1, (int)std::ceil((hi[i] - lo[i]) / AGB_CELL));
+    }
+}
+size_t cell_grid_size(const ag_problem *p)
+{
+    int nc[3];
+    double lo[3], hi[3];
+    cell_grid(p, nc, lo, hi);
+    return (size_t)nc[0] * nc[1] * nc[2];
 }
 
 // Build the device image of a problem (host work is O(atoms + tables)).
@@ -452,8 +535,30 @@ ag_status build_plan(ag_plan *pl, const ag_problem *p, cudaStream_t s, bool pipe
     // table, the chunking and the partial sums.  A slab-pipelined one-shot run
     // launches its first far-field slab from here, so that the GPU computes
     // while the rest of the plan is built on the host.
-    std::vector<double> x(N), y(N), z(N), x128(N), y128(N), z128(N);
-    std::vector<float> qw(N);
+    //
+    // The kernels' tables are packed by kernels where the tables are on the
+    // device already, and in one-shot calls, whose caller waits (41^3 points:
+    // 359 us against 469 with the tables packed on the host and an upload for
+    // each array).  Plans pack them on the host: those of a batch are built
+    // while the GPU is full of earlier instances' persistent blocks, and a
+    // packing kernel would wait for them (24 instances one-shot: 26.9 ms
+    // against 23.1).
+    const bool dev_pack = dev_tables || !pl->own;
+    const int nT = std::max(1, p->n_rec_types);
+    const size_t vdw_n = (nAM > 0 && dev_pack && !dev_tables) ? (size_t)p->n_rec_types * nAM * AG_NEINT : 0;
+    const size_t cells = cell_grid_size(p);
+    const size_t early_bytes = (size_t)N * 28 + 2 * AG_NDIEL * sizeof(double);
+    const size_t late_bytes = (size_t)N * 168 + (cells + 1) * sizeof(int) + vdw_n * sizeof(float) +
+                              (size_t)AG_NDIEL * 16 + 8192;
+    constexpr int kEarly = 8, kLate = 32;
+    char *pinned = nullptr;  // for one-shot calls, which share the context's buffers too
+    if (!pl->own) AGB_CK(pl->ctx->stage(Stage::room(early_bytes, kEarly) + Stage::room(late_bytes, kLate), s, &pinned));
+    Stage early(early_bytes, kEarly, pinned);
+    Stage late(late_bytes, kLate, pinned ? pinned + Stage::room(early_bytes, kEarly) : nullptr);
+    double *x128 = early.make(N, &pl->x128), *y128 = early.make(N, &pl->y128), *z128 = early.make(N, &pl->z128);
+    float *qw = early.make(N, &pl->qw);
+    double *dx, *dy, *dz, *dsolfn = nullptr, *deps = nullptr;
+    double *x = late.make(N, &dx), *y = late.make(N, &dy), *z = late.make(N, &dz);
     for (int a = 0; a < N; a++) {
         x[a] = p->coord[3 * a]; y[a] = p->coord[3 * a + 1]; z[a] = p->coord[3 * a + 2];
         x128[a] = x[a] * AG_A_DIV; y128[a] = y[a] * AG_A_DIV; z128[a] = z[a] * AG_A_DIV;
@@ -489,21 +594,22 @@ ag_status build_plan(ag_plan *pl, const ag_problem *p, cudaStream_t s, bool pipe
             pl->tab_len = AG_NDIEL;
         }
     }
-    const int TL = pl->tab_len;
     std::vector<float> far_tab;
     if (!dev_tables) {
-        // [0, tab_len): the far kernel's table, zero below FAR_BIN0 (those
-        // pairs are the near kernel's), bin NDIEL-1 repeated past it;
-        // [tab_len, tab_len + NDIEL): the whole table, for far pairs whose
-        // exact bin the bin guard finds below FAR_BIN0
-        far_tab.assign((size_t)TL + AG_NDIEL, 0.f);
-        for (int k = 0; k < AG_NDIEL; k++) far_tab[TL + k] = (float)(p->dddiel ? p->r_epsilon_fn[k] : p->invdielcal);
-        for (int k = AG_NEINT; k < TL; k++) far_tab[k] = far_tab[TL + std::min(k, AG_NDIEL - 1)];
+        early.add(p->sol_fn, AG_NDIEL, &dsolfn);
+        if (dev_pack && p->dddiel) early.add(p->r_epsilon_fn, AG_NDIEL, &deps);
         // a constant dielectric needs no far-field table gather
         if (!p->dddiel) {
             pl->far_mode = FAR_TAB_CONST;
             pl->far_const = (float)p->invdielcal;
         }
+    }
+    if (!dev_pack) {
+        // as k_pack_lines does
+        const int TL = pl->tab_len;
+        far_tab.assign((size_t)TL + AG_NDIEL, 0.f);
+        for (int k = 0; k < AG_NDIEL; k++) far_tab[TL + k] = (float)(p->dddiel ? p->r_epsilon_fn[k] : p->invdielcal);
+        for (int k = AG_NEINT; k < TL; k++) far_tab[k] = far_tab[TL + std::min(k, AG_NDIEL - 1)];
     }
     // far-field chunking: units of at least kFarMinChunk atoms, enough for 4
     // waves of CTAs per launch; a slab-pipelined one-shot run launches one slab
@@ -541,11 +647,35 @@ ag_status build_plan(ag_plan *pl, const ag_problem *p, cudaStream_t s, bool pipe
         AGB_CK(B->ensure("edge_bits", far_edge_bits_bytes(pl->n_chunks, pl->chunk_atoms, nframes), &v));
         pl->edge_bits = (uint32_t *)v;
     }
-    AGB_CK(upload(B, "x128", x128.data(), N, &pl->x128, s, acc));
-    AGB_CK(upload(B, "y128", y128.data(), N, &pl->y128, s, acc));
-    AGB_CK(upload(B, "z128", z128.data(), N, &pl->z128, s, acc));
-    AGB_CK(upload(B, "qw", qw.data(), N, &pl->qw, s, acc));
-    if (!dev_tables) AGB_CK(upload(B, "far_tab", far_tab.data(), far_tab.size(), &pl->far_tab, s, acc));
+    AGB_CK(early.send(B, "far_inputs", s, acc));
+    // the far kernel's table (zero below FAR_BIN0, whose pairs are the near
+    // kernel's, bin NDIEL-1 repeated up to tab_len; then the whole table, for
+    // far pairs whose exact bin the bin guard finds below FAR_BIN0), the near
+    // e table, the desolvation table and the FP64 dielectric table
+    double *dreps;
+    if (dev_pack) {
+        AGB_CK(B->ensure("far_tab", ((size_t)pl->tab_len + AG_NDIEL) * sizeof(float), &v)); pl->far_tab = (float *)v;
+        AGB_CK(B->ensure("etab", AG_NDIEL * sizeof(float), &v)); pl->etab = (float *)v;
+        AGB_CK(B->ensure("solf", AG_NDIEL * sizeof(float), &v)); pl->solf = (float *)v;
+        AGB_CK(B->ensure("reps", AG_NDIEL * sizeof(double), &v)); dreps = (double *)v;
+        if (dev_tables) {
+            AGB_CK(B->ensure("sol_fn", AG_NDIEL * sizeof(double), &v)); dsolfn = (double *)v;
+            AGB_CK(cudaMemcpyAsync(dsolfn, p->sol_fn, AG_NDIEL * sizeof(double), cudaMemcpyDeviceToDevice, s));
+        }
+        AGB_CK(launch_pack_lines(dsolfn, !p->dddiel ? nullptr : dev_tables ? p->r_epsilon_fn : deps, p->dddiel,
+                                 p->invdielcal, p->coeff_estat, pl->far_tab, pl->tab_len, pl->etab, pl->solf, dreps, s));
+    } else {
+        AGB_CK(upload(B, "far_tab", far_tab.data(), far_tab.size(), &pl->far_tab, s));
+        *acc += far_tab.size() * sizeof(float);
+        float *etab = late.make(AG_NDIEL, &pl->etab), *solf = late.make(AG_NDIEL, &pl->solf);
+        double *reps = late.make(AG_NDIEL, &dreps);
+        for (int k = 0; k < AG_NDIEL; k++) {
+            const double f = p->dddiel ? p->r_epsilon_fn[k] : p->invdielcal;
+            reps[k] = p->dddiel ? f : 0.0;
+            etab[k] = (float)(f * p->coeff_estat);
+            solf[k] = (float)p->sol_fn[k];
+        }
+    }
     pl->far_early = 0;
     if (pipelined && early_far && !dev_tables && pl->far_partial && d.elec_map >= 0) {
         // the run's statistics start here: counters cleared, then ev0, then the fork
@@ -559,8 +689,8 @@ ag_status build_plan(ag_plan *pl, const ag_problem *p, cudaStream_t s, bool pipe
 
     // the near kernel's staged atom record: bond vectors + vol, lone-pair
     // normal + desolvation factor, and packed metadata (type, hbond, rexp, flags)
-    std::vector<float4> atomA(std::max(N, 1)), atomB(std::max(N, 1));
-    std::vector<int> meta(std::max(N, 1), 0);
+    float4 *atomA = late.make(N, &pl->atomA), *atomB = late.make(N, &pl->atomB);
+    int *meta = late.make(N, &pl->meta);
     for (int a = 0; a < N; a++) {
         const double *rv = p->rvector + 3 * a, *rv2 = p->rvector2 + 3 * a;
         atomA[a] = make_float4((float)rv[0], (float)rv[1], (float)rv[2], (float)p->vol[a]);
@@ -577,15 +707,11 @@ ag_status build_plan(ag_plan *pl, const ag_problem *p, cudaStream_t s, bool pipe
         if (p->hbond[a] == 1 || p->hbond[a] == 2) h_index.push_back(a);
 
     // cell list over the grid box grown by the near radius
-    const double rc = AGB_NEAR_RADIUS, cs = AGB_CELL;
+    const double cs = AGB_CELL;
     double lo[3], hi[3];
     int nc[3];
-    for (int i = 0; i < 3; i++) {
-        lo[i] = (double)(-p->ne[i]) * p->spacing - rc;
-        hi[i] = (double)(p->n1[i] - 1 - p->ne[i]) * p->spacing + rc;
-        nc[i] = std::max(1, (int)std::ceil((hi[i] - lo[i]) / cs));
-        d.cell0[i] = lo[i];
-    }
+    cell_grid(p, nc, lo, hi);
+    for (int i = 0; i < 3; i++) d.cell0[i] = lo[i];
     d.ncx = nc[0]; d.ncy = nc[1]; d.ncz = nc[2];
     d.cell_size = cs;
     const size_t ncell = (size_t)nc[0] * nc[1] * nc[2];
@@ -693,97 +819,10 @@ ag_status build_plan(ag_plan *pl, const ag_problem *p, cudaStream_t s, bool pipe
     // tables: vdW/H-bond transposed to [type][bin][column], columns in kernel order
     // (whole 32-byte rows of 8 columns)
     pl->mpad = pl->groups.back().col0 + std::max(8, (pl->groups.back().ng + 7) / 8 * 8);
-    const int nT = std::max(1, p->n_rec_types);
     std::vector<int> colmap(pl->mpad, -1);
     for (const NearGroup &g : pl->groups)
         for (int k = 0; k < g.ng; k++)
             if (!skip_map[g.out_map[k]]) colmap[g.col0 + k] = g.out_map[k];
-    std::vector<float> vdwT, etab, solf;
-    std::vector<double> reps;
-    if (!dev_tables) {
-        vdwT.assign((size_t)nT * AG_NEINT * pl->mpad, 0.f);
-        for (int c = 0; c < pl->mpad; c++) {
-            const int m = colmap[c];
-            if (m < 0) continue;
-            for (int t = 0; t < p->n_rec_types; t++)
-                for (int b = 0; b < AG_NEINT; b++)
-                    vdwT[((size_t)t * AG_NEINT + b) * pl->mpad + c] = p->e_vdw_hb[((size_t)t * nAM + m) * AG_NEINT + b];
-        }
-        etab.resize(AG_NDIEL);
-        solf.resize(AG_NDIEL);
-        reps.assign(AG_NDIEL, 0.0);
-        for (int k = 0; k < AG_NDIEL; k++) {
-            const double f = p->dddiel ? p->r_epsilon_fn[k] : p->invdielcal;
-            if (p->dddiel) reps[k] = p->r_epsilon_fn[k];
-            etab[k] = (float)(f * p->coeff_estat);
-            solf[k] = (float)p->sol_fn[k];
-        }
-    }
-
-    // uploads
-    double *dx, *dy, *dz, *dq, *dvol, *dsol, *drv, *drv2;
-    int *dtype, *dhb, *drexp, *dh, *dcs, *dca, *dmc, *dmh, *dmhb;
-    uint8_t *ddis;
-    double *dms, *dmv, *dsolfn, *dreps;
-    AGB_CK(upload(B, "x", x.data(), N, &dx, s, acc));
-    AGB_CK(upload(B, "y", y.data(), N, &dy, s, acc));
-    AGB_CK(upload(B, "z", z.data(), N, &dz, s, acc));
-    AGB_CK(upload(B, "q", p->charge, N, &dq, s, acc));
-    AGB_CK(upload(B, "vol", p->vol, N, &dvol, s, acc));
-    AGB_CK(upload(B, "solpar", p->solpar, N, &dsol, s, acc));
-    AGB_CK(upload(B, "rv", p->rvector, 3 * (size_t)N, &drv, s, acc));
-    AGB_CK(upload(B, "rv2", p->rvector2, 3 * (size_t)N, &drv2, s, acc));
-    AGB_CK(upload(B, "type", p->rec_type, N, &dtype, s, acc));
-    AGB_CK(upload(B, "hbond", p->hbond, N, &dhb, s, acc));
-    AGB_CK(upload(B, "rexp", p->rexp, N, &drexp, s, acc));
-    AGB_CK(upload(B, "disorder", p->disorder, N, &ddis, s, acc));
-    AGB_CK(upload(B, "atomA", atomA.data(), atomA.size(), &pl->atomA, s, acc));
-    AGB_CK(upload(B, "atomB", atomB.data(), atomB.size(), &pl->atomB, s, acc));
-    AGB_CK(upload(B, "meta", meta.data(), meta.size(), &pl->meta, s, acc));
-    AGB_CK(upload(B, "h_index", h_index.data(), h_index.size(), &dh, s, acc));
-    AGB_CK(upload(B, "cell_start", cell_start.data(), cell_start.size(), &dcs, s, acc));
-    AGB_CK(upload(B, "cell_atoms", cell_atoms.data(), cell_atoms.size(), &dca, s, acc));
-    std::vector<int> mc(std::max(nAM, 1), 0), mh(std::max(nAM, 1), 0), mhb(std::max(nAM, 1), 0);
-    std::vector<double> ms(std::max(nAM, 1), 0.0), mv(std::max(nAM, 1), 0.0);
-    for (int m = 0; m < nAM; m++) {
-        mc[m] = p->map_is_covalent[m]; mh[m] = p->map_is_hbonder[m]; mhb[m] = p->map_hbond[m];
-        ms[m] = p->map_solpar_probe[m]; mv[m] = p->map_vol_probe[m];
-    }
-    AGB_CK(upload(B, "m_cov", mc.data(), mc.size(), &dmc, s, acc));
-    AGB_CK(upload(B, "m_hb", mh.data(), mh.size(), &dmh, s, acc));
-    AGB_CK(upload(B, "m_hbond", mhb.data(), mhb.size(), &dmhb, s, acc));
-    AGB_CK(upload(B, "m_solpar", ms.data(), ms.size(), &dms, s, acc));
-    AGB_CK(upload(B, "m_vol", mv.data(), mv.size(), &dmv, s, acc));
-    if (!dev_tables) {
-        AGB_CK(upload(B, "vdwT", vdwT.data(), vdwT.size(), &pl->vdwT, s, acc));
-        AGB_CK(upload(B, "etab", etab.data(), etab.size(), &pl->etab, s, acc));
-        AGB_CK(upload(B, "solf", solf.data(), solf.size(), &pl->solf, s, acc));
-        AGB_CK(upload(B, "sol_fn", p->sol_fn, AG_NDIEL, &dsolfn, s, acc));
-        AGB_CK(upload(B, "reps", reps.data(), reps.size(), &dreps, s, acc));
-    } else {
-        // tables already on the device (e.g. from ag_tables_build): packed by kernels
-        int *dcol;
-        void *vv;
-        AGB_CK(upload(B, "colmap", colmap.data(), colmap.size(), &dcol, s, acc));
-        AGB_CK(B->ensure("vdwT", (size_t)nT * AG_NEINT * pl->mpad * sizeof(float), &vv)); pl->vdwT = (float *)vv;
-        AGB_CK(B->ensure("far_tab", ((size_t)pl->tab_len + AG_NDIEL) * sizeof(float), &vv)); pl->far_tab = (float *)vv;
-        AGB_CK(B->ensure("etab", AG_NDIEL * sizeof(float), &vv)); pl->etab = (float *)vv;
-        AGB_CK(B->ensure("solf", AG_NDIEL * sizeof(float), &vv)); pl->solf = (float *)vv;
-        AGB_CK(B->ensure("sol_fn", AG_NDIEL * sizeof(double), &vv)); dsolfn = (double *)vv;
-        AGB_CK(B->ensure("reps", AG_NDIEL * sizeof(double), &vv)); dreps = (double *)vv;
-        AGB_CK(cudaMemcpyAsync(dsolfn, p->sol_fn, AG_NDIEL * sizeof(double), cudaMemcpyDeviceToDevice, s));
-        AGB_CK(cudaMemsetAsync(pl->vdwT, 0, (size_t)nT * AG_NEINT * pl->mpad * sizeof(float), s));
-        AGB_CK(launch_pack_tables(p->e_vdw_hb, p->n_rec_types, nAM, dcol, pl->mpad, pl->vdwT, p->sol_fn,
-                                  p->dddiel ? p->r_epsilon_fn : nullptr, p->dddiel, p->invdielcal, p->coeff_estat,
-                                  pl->far_tab, pl->tab_len, pl->etab, pl->solf, dreps, s));
-    }
-
-    d.x = dx; d.y = dy; d.z = dz; d.q = dq; d.vol = dvol; d.solpar = dsol; d.rv = drv; d.rv2 = drv2;
-    d.type = dtype; d.hbond = dhb; d.rexp = drexp; d.disorder = ddis;
-    d.n_h = (int)h_index.size(); d.h_index = dh;
-    d.cell_start = dcs; d.cell_atoms = dca;
-    d.m_cov = dmc; d.m_hb = dmh; d.m_hbond = dmhb; d.m_solpar = dms; d.m_vol = dmv;
-    d.vdw = pl->vdwT; d.sol_fn = dsolfn; d.reps = dreps; d.far_tab = pl->far_tab;
 
     // outputs and scratch
     pl->floating = p->floating_grid ? 1 : 0;
@@ -809,20 +848,61 @@ ag_status build_plan(ag_plan *pl, const ag_problem *p, cudaStream_t s, bool pipe
     } else {
         pl->cov = nullptr;
     }
+    pl->d_reduce = nullptr;
+    pl->d_reduce_begin = nullptr;
     if (pl->far_partial && d.elec_map >= 0) {
         const ReduceInst r{d.P, pl->n_chunks, pl->far_partial, pl->maps32 + (size_t)d.elec_map * P};
         const long long beg[2] = {0, d.P};
-        AGB_CK(B->ensure("reduce", sizeof r, &v));
-        pl->d_reduce = (ReduceInst *)v;
-        AGB_CK(B->ensure("reduce_begin", sizeof beg, &v));
-        pl->d_reduce_begin = (long long *)v;
-        AGB_CK(cudaMemcpyAsync(pl->d_reduce, &r, sizeof r, cudaMemcpyHostToDevice, s));
-        AGB_CK(cudaMemcpyAsync(pl->d_reduce_begin, beg, sizeof beg, cudaMemcpyHostToDevice, s));
-        AGB_CK(cudaStreamSynchronize(s));  // sources are locals
-    } else {
-        pl->d_reduce = nullptr;
-        pl->d_reduce_begin = nullptr;
+        late.add(&r, 1, &pl->d_reduce);
+        late.add(beg, 2, &pl->d_reduce_begin);
     }
+
+    // uploads: the rest of the inputs in one copy
+    double *dq, *dvol, *dsol, *drv, *drv2;
+    int *dtype, *dhb, *drexp, *dh, *dcs, *dca, *dcol;
+    uint8_t *ddis;
+    float *dvdw = nullptr;
+    late.add(p->charge, N, &dq);
+    late.add(p->vol, N, &dvol);
+    late.add(p->solpar, N, &dsol);
+    late.add(p->rvector, 3 * (size_t)N, &drv);
+    late.add(p->rvector2, 3 * (size_t)N, &drv2);
+    late.add(p->rec_type, N, &dtype);
+    late.add(p->hbond, N, &dhb);
+    late.add(p->rexp, N, &drexp);
+    late.add(p->disorder, N, &ddis);
+    late.add(h_index.data(), h_index.size(), &dh);
+    late.add(cell_start.data(), cell_start.size(), &dcs);
+    late.add(cell_atoms.data(), cell_atoms.size(), &dca);
+    late.add(colmap.data(), colmap.size(), &dcol);
+    if (vdw_n) late.add(p->e_vdw_hb, vdw_n, &dvdw);
+    AGB_CK(late.send(B, "inputs", s, acc));
+    // vdW/H-bond tables transposed to [type][bin][column]
+    const size_t vdwT_n = (size_t)nT * AG_NEINT * pl->mpad;
+    std::vector<float> vdwT;
+    if (dev_pack && nAM > 0 && p->n_rec_types > 0) {
+        AGB_CK(B->ensure("vdwT", vdwT_n * sizeof(float), &v));
+        pl->vdwT = (float *)v;
+        AGB_CK(launch_pack_vdw(dev_tables ? p->e_vdw_hb : dvdw, p->n_rec_types, nAM, dcol, pl->mpad, pl->vdwT, s));
+    } else {
+        vdwT.assign(vdwT_n, 0.f);
+        for (int c = 0; c < pl->mpad; c++) {
+            const int m = colmap[c];
+            if (m < 0) continue;
+            for (int t = 0; t < p->n_rec_types; t++)
+                for (int b = 0; b < AG_NEINT; b++)
+                    vdwT[((size_t)t * AG_NEINT + b) * pl->mpad + c] = p->e_vdw_hb[((size_t)t * nAM + m) * AG_NEINT + b];
+        }
+        AGB_CK(upload(B, "vdwT", vdwT.data(), vdwT_n, &pl->vdwT, s));
+        *acc += vdwT_n * sizeof(float);
+    }
+
+    d.x = dx; d.y = dy; d.z = dz; d.q = dq; d.vol = dvol; d.solpar = dsol; d.rv = drv; d.rv2 = drv2;
+    d.type = dtype; d.hbond = dhb; d.rexp = drexp; d.disorder = ddis;
+    d.n_h = (int)h_index.size(); d.h_index = dh;
+    d.cell_start = dcs; d.cell_atoms = dca;
+    d.vdw = pl->vdwT; d.sol_fn = dsolfn; d.reps = dreps; d.far_tab = pl->far_tab;
+    if (!pinned || !vdwT.empty()) AGB_CK(cudaStreamSynchronize(s));  // sources are locals
     return AG_OK;
 }
 
@@ -1433,6 +1513,7 @@ ag_status ag_context_destroy(ag_context *ctx)
     if (ctx->evn1) cudaEventDestroy(ctx->evn1);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     if (ctx->h_text) cudaFreeHost(ctx->h_text);
+    if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
     for (cudaEvent_t e : ctx->tev)
         if (e) cudaEventDestroy(e);
     delete ctx;
@@ -1754,13 +1835,13 @@ ag_status ag_tables_build(ag_context *ctx, const ag_table_params *tp, float *e_v
     const size_t npar = (size_t)nT * nAM;
     double *dcA, *dcB, *dR, *dE;
     int *dxA, *dxB, *dcov, *dbad;
-    AGB_CK(upload(&B, "cA", tp->cA, npar, &dcA, s, nullptr));
-    AGB_CK(upload(&B, "cB", tp->cB, npar, &dcB, s, nullptr));
-    AGB_CK(upload(&B, "Rij", tp->Rij, npar, &dR, s, nullptr));
-    AGB_CK(upload(&B, "epsij", tp->epsij, npar, &dE, s, nullptr));
-    AGB_CK(upload(&B, "xA", tp->xA, npar, &dxA, s, nullptr));
-    AGB_CK(upload(&B, "xB", tp->xB, npar, &dxB, s, nullptr));
-    AGB_CK(upload(&B, "cov", tp->map_is_covalent, (size_t)nAM, &dcov, s, nullptr));
+    AGB_CK(upload(&B, "cA", tp->cA, npar, &dcA, s));
+    AGB_CK(upload(&B, "cB", tp->cB, npar, &dcB, s));
+    AGB_CK(upload(&B, "Rij", tp->Rij, npar, &dR, s));
+    AGB_CK(upload(&B, "epsij", tp->epsij, npar, &dE, s));
+    AGB_CK(upload(&B, "xA", tp->xA, npar, &dxA, s));
+    AGB_CK(upload(&B, "xB", tp->xB, npar, &dxB, s));
+    AGB_CK(upload(&B, "cov", tp->map_is_covalent, (size_t)nAM, &dcov, s));
     a.cA = dcA; a.cB = dcB; a.Rij = dR; a.epsij = dE; a.xA = dxA; a.xB = dxB; a.map_is_covalent = dcov;
     void *v;
     AGB_CK(B.ensure("bad", sizeof(int), &v)); dbad = (int *)v;

@@ -192,9 +192,6 @@ struct DevProblem {
     double cell0[3], cell_size;        // origin (centred frame), edge
     const int *cell_start;             // [ncx*ncy*ncz + 1]
     const int *cell_atoms;             // [n_near] file indices sorted by cell
-    // per-map constants
-    const int *m_cov, *m_hb, *m_hbond;
-    const double *m_solpar, *m_vol;
     // tables
     const float *vdw;                  // [types][atom_maps][NEINT]
     const double *sol_fn, *reps;       // [NDIEL]

@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(kThreads) k_sol_eps(TableArgs a, double *sol_f
     }
 }
 
-// Plan tables from device-resident problem tables: vdwT [type][bin][mpad]
+// Plan tables from a problem's tables in device memory: vdwT [type][bin][mpad]
 // (column c holds map colmap[c], or zeros), far_tab [tab_len + NDIEL] (the
 // far kernel's table: zero below FAR_BIN0, bin NDIEL-1 repeated up to
 // tab_len; then the whole table) / etab / solf (FP32) and
@@ -170,13 +170,18 @@ cudaError_t launch_tables_build(const TableArgs &a, float *raw, float *e_vdw_hb,
     return cudaGetLastError();
 }
 
-cudaError_t launch_pack_tables(const float *e_vdw_hb, int n_rec_types, int n_atom_maps, const int *colmap, int mpad,
-                               float *vdwT, const double *sol_fn, const double *r_eps, int dddiel, double invdielcal,
-                               double coeff_estat, float *far_tab, int tab_len, float *etab, float *solf,
-                               double *reps, cudaStream_t s)
+cudaError_t launch_pack_vdw(const float *e_vdw_hb, int n_rec_types, int n_atom_maps, const int *colmap, int mpad,
+                            float *vdwT, cudaStream_t s)
 {
     const long long n = (long long)n_rec_types * AG_NEINT * mpad;
     if (n > 0) k_pack_vdw<<<blocks_for(n), kThreads, 0, s>>>(e_vdw_hb, n_rec_types, n_atom_maps, colmap, mpad, vdwT);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_pack_lines(const double *sol_fn, const double *r_eps, int dddiel, double invdielcal,
+                              double coeff_estat, float *far_tab, int tab_len, float *etab, float *solf, double *reps,
+                              cudaStream_t s)
+{
     k_pack_lines<<<blocks_for(std::max(AG_NDIEL, tab_len)), kThreads, 0, s>>>(sol_fn, r_eps, dddiel, invdielcal,
                                                                                coeff_estat, far_tab, tab_len, etab,
                                                                                solf, reps);

@@ -18,11 +18,12 @@ struct TableArgs {
 // fatal parameter (NaN coefficient or zero exponent).
 cudaError_t launch_tables_build(const TableArgs &a, float *raw, float *e_vdw_hb, double *sol_fn, double *r_eps,
                                 int *bad, cudaStream_t s);
-// Plan tables from device-resident problem tables (colmap [mpad]: map of each
-// vdW column, -1 for none).
-cudaError_t launch_pack_tables(const float *e_vdw_hb, int n_rec_types, int n_atom_maps, const int *colmap, int mpad,
-                               float *vdwT, const double *sol_fn, const double *r_eps, int dddiel, double invdielcal,
-                               double coeff_estat, float *far_tab, int tab_len, float *etab, float *solf,
-                               double *reps, cudaStream_t s);
+// Plan tables from a problem's tables in device memory (colmap [mpad]: map of
+// each vdW column, -1 for none).
+cudaError_t launch_pack_vdw(const float *e_vdw_hb, int n_rec_types, int n_atom_maps, const int *colmap, int mpad,
+                            float *vdwT, cudaStream_t s);
+cudaError_t launch_pack_lines(const double *sol_fn, const double *r_eps, int dddiel, double invdielcal,
+                              double coeff_estat, float *far_tab, int tab_len, float *etab, float *solf, double *reps,
+                              cudaStream_t s);
 
 }  // namespace agb
