@@ -462,18 +462,18 @@ struct Stage {
 // Error bounds of the canonical FP32 distances for a grid spacing (in bins):
 // the far kernel's bin-guard multipliers and the near kernel's guard, from the
 // largest frame-relative point coordinate and whether every frame point
-// coordinate il*spacing_adiv is an exact float.  rsqrt.approx.f32 is taken at
+// coordinate il*spacing_adiv is an exact float (il up to half a frame).  rsqrt.approx.f32 is taken at
 // 2.5 * 2^-24 relative error (PTX ISA: 2^-22.9 = 2.14 * 2^-24; checked on the
 // device by ag_diag_rsqrt_error).
 void far_guard(double spacing_adiv, float *lo, float *hi, float *near)
 {
     bool exact = true;
-    for (int il = 0; il < FRAME_X; il++) {
+    for (int il = 0; il <= FRAME_X / 2; il++) {
         const double v = (double)il * spacing_adiv;
         exact &= std::fma((double)il, spacing_adiv, -v) == 0.0 && (double)(float)v == v;
     }
-    const double px = (FRAME_X - 1) * spacing_adiv, pyz = (FRAME_Y - 1) * spacing_adiv;
-    const double p_max = std::sqrt(px * px + 2 * pyz * pyz);
+    const double px = FRAME_X / 2 * spacing_adiv, py = FRAME_Y / 2 * spacing_adiv, pz = FRAME_Z / 2 * spacing_adiv;
+    const double p_max = std::sqrt(px * px + py * py + pz * pz);
     far_edge_multipliers(p_max, exact, 2.5, lo, hi);
     *near = near_edge_guard(p_max, exact, 2.5);
 }

@@ -27,7 +27,7 @@ constexpr float FAR_MAX_T = (float)(AG_NDIEL - 1);
 constexpr float FAR_CLAMP_T = (float)(AG_NDIEL - 1) + 0.5f;
 constexpr uint32_t MAGIC_BITS = 0x4B000000u;  // bits of 2^23: bits(2^23 + k) = MAGIC_BITS + k, 0 <= k < 2^23
 
-// Frame origin in bins: ((o - ne) * spacing) * A_DIV, formed like the
+// Frame origin (the grid point o of the frame) in bins: ((o - ne) * spacing) * A_DIV, formed like the
 // reference forms a grid coordinate (main.cpp:2859); the scaling by A_DIV = 2^7
 // is exact, so this equals ((o - ne) * (spacing * A_DIV)).
 __host__ __device__ inline double frame_origin_bins(int o, int ne, double spacing_adiv)
@@ -139,17 +139,23 @@ constexpr int FAR_TAB_MAX = 16384;
 // FP32 distance t of a far pair (t >= FAR_T0 bins), rounded up so that 1 - d
 // and 1 + d are floats.  With D the exact frame-relative distance (bins), A
 // the atom's and P the point's frame-relative coordinates (|A| <= |D| + |P|):
+// (the far and near kernels' count from the frame's middle, point FRAME_X/2
+// and so on, which halves |P|):
 //   coordinates rounded to FP32 and dx = A - P rounded:
 //       |error vector| <= 2^-24 (|A| + |D| + |P| [P inexact]) <= 2^-24 (2|D| + (1 + [P inexact])|P|)
 //   t2 = dx^2 + (dy^2 + dz^2) by two FMAs: relative 3 * 2^-24, 1.5 * 2^-24 on t
 //   rsqrt.approx: relative rho;  t = t2 * rs rounded: 2^-24
 // so |t/D - 1| <= 2^-24 (4.5 + (1 + [P inexact]) |P|max / FAR_T0) + rho.
+// 1.005 covers the terms of second order, below 1e-5 of this.  Whole units of
+// 2^-24 count: at 48 bins between points they are 8 on each side; from the
+// frame's corner and with a margin of 1/16 they were 10, which flags 25% more
+// pairs.
 // rho_ulps is rho in units of 2^-24; p_max the largest |P| of a frame point;
 // p_exact whether every frame point coordinate is an exact float.
 __host__ inline void far_edge_multipliers(double p_max, bool p_exact, double rho_ulps, float *lo, float *hi)
 {
     const double u = 1.0 / 16777216.0;  // 2^-24
-    const double d = u * (4.5 + rho_ulps + (p_exact ? 1.0 : 2.0) * p_max / (double)FAR_T0) * 1.0625;
+    const double d = u * (4.5 + rho_ulps + (p_exact ? 1.0 : 2.0) * p_max / (double)FAR_T0) * 1.005;
     const double kl = std::ceil(d / u), kh = std::ceil(d / (2 * u));
     *lo = (float)(1.0 - kl * u);        // floats below 1 are spaced 2^-24
     *hi = (float)(1.0 + kh * 2 * u);    // floats above 1 are spaced 2^-23

@@ -149,21 +149,21 @@ __device__ __forceinline__ void far_unit_n(const FarArgs &a, int f, int chunk, c
     const int tid = threadIdx.x, lane = tid & 31, v = (tid >> 5) & 3, half = tid / EF_GROUP;
     const int fx = f % a.nfx, fy = (f / a.nfx) % a.nfy, fz = f / (a.nfx * a.nfy);
     const int ox = fx * FRAME_X, oy = fy * FRAME_Y, oz = fz * FRAME_Z;
-    // frame origin in bins, exactly (ox-nex)*spacing*A_DIV as the reference forms c (main.cpp:2859)
-    const double X0 = frame_origin_bins(ox, a.nex, a.spacing_adiv);
-    const double Y0 = frame_origin_bins(oy, a.ney, a.spacing_adiv);
-    const double Z0 = frame_origin_bins(oz, a.nez, a.spacing_adiv);
+    // the frame's middle in bins, exactly (x-nex)*spacing*A_DIV as the reference forms c (main.cpp:2859)
+    const double X0 = frame_origin_bins(ox + FRAME_X / 2, a.nex, a.spacing_adiv);
+    const double Y0 = frame_origin_bins(oy + FRAME_Y / 2, a.ney, a.spacing_adiv);
+    const double Z0 = frame_origin_bins(oz + FRAME_Z / 2, a.nez, a.spacing_adiv);
     // lane footprint 4x4x2 (fewest table bank conflicts): x = tx + 8j and tx + 8j + 4
     const int tx = lane & 3, ty = (lane >> 2) & 3, tz = (lane >> 4) + 2 * v;
     const bool warp_in = oz + 2 * v < a.n1z;
-    const float npz = -frame_point_coord(tz, a.spacing_adiv) * FAR_DOWN;
-    const float2 npy = make_float2(-frame_point_coord(ty, a.spacing_adiv) * FAR_DOWN,
-                                   -frame_point_coord(ty + 4, a.spacing_adiv) * FAR_DOWN);
+    const float npz = -frame_point_coord(tz - FRAME_Z / 2, a.spacing_adiv) * FAR_DOWN;
+    const float2 npy = make_float2(-frame_point_coord(ty - FRAME_Y / 2, a.spacing_adiv) * FAR_DOWN,
+                                   -frame_point_coord(ty + 4 - FRAME_Y / 2, a.spacing_adiv) * FAR_DOWN);
     float2 npx[NJ];
 #pragma unroll
     for (int j = 0; j < NJ; j++)
-        npx[j] = make_float2(-frame_point_coord(tx + 8 * j, a.spacing_adiv) * FAR_DOWN,
-                             -frame_point_coord(tx + 8 * j + 4, a.spacing_adiv) * FAR_DOWN);
+        npx[j] = make_float2(-frame_point_coord(tx + 8 * j - FRAME_X / 2, a.spacing_adiv) * FAR_DOWN,
+                             -frame_point_coord(tx + 8 * j + 4 - FRAME_X / 2, a.spacing_adiv) * FAR_DOWN);
     float2 tot[ROWS][NJ];
 #pragma unroll
     for (int r = 0; r < ROWS; r++)
@@ -460,20 +460,20 @@ __device__ __forceinline__ void far_fix_unit(const FarArgs &a, int f, int chunk,
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int fx = f % a.nfx, fy = (f / a.nfx) % a.nfy, fz = f / (a.nfx * a.nfy);
     const int ox = fx * FRAME_X, oy = fy * FRAME_Y, oz = fz * FRAME_Z;
-    const double X0 = frame_origin_bins(ox, a.nex, a.spacing_adiv);
-    const double Y0 = frame_origin_bins(oy, a.ney, a.spacing_adiv);
-    const double Z0 = frame_origin_bins(oz, a.nez, a.spacing_adiv);
+    const double X0 = frame_origin_bins(ox + FRAME_X / 2, a.nex, a.spacing_adiv);
+    const double Y0 = frame_origin_bins(oy + FRAME_Y / 2, a.ney, a.spacing_adiv);
+    const double Z0 = frame_origin_bins(oz + FRAME_Z / 2, a.nez, a.spacing_adiv);
     const FarLane L = far_lane(a, tid, oy, oz);
     const bool point_in = oy + L.ty < a.n1y && oz + L.tz < a.n1z;
     __syncthreads();  // the previous unit (batch kernel) is done with S
 #pragma unroll
     for (int j = 0; j < EF_PAIRS; j++) {
-        S.npx[j][tid] = make_float2(-frame_point_coord(L.tx + 8 * j, a.spacing_adiv),
-                                    -frame_point_coord(L.tx + 8 * j + 4, a.spacing_adiv));
+        S.npx[j][tid] = make_float2(-frame_point_coord(L.tx + 8 * j - FRAME_X / 2, a.spacing_adiv),
+                                    -frame_point_coord(L.tx + 8 * j + 4 - FRAME_X / 2, a.spacing_adiv));
         S.corr[2 * j][tid] = 0ull;
         S.corr[2 * j + 1][tid] = 0ull;
     }
-    S.npyz[tid] = make_float2(-frame_point_coord(L.ty, a.spacing_adiv), -frame_point_coord(L.tz, a.spacing_adiv));
+    S.npyz[tid] = make_float2(-frame_point_coord(L.ty - FRAME_Y / 2, a.spacing_adiv), -frame_point_coord(L.tz - FRAME_Z / 2, a.spacing_adiv));
     if (tid < FRAME_X + FRAME_Y + FRAME_Z) {
         const int i = tid < FRAME_X ? ox + tid - a.nex
                     : tid < FRAME_X + FRAME_Y ? oy + (tid - FRAME_X) - a.ney : oz + (tid - FRAME_X - FRAME_Y) - a.nez;
@@ -654,12 +654,12 @@ __global__ void __launch_bounds__(256) k_far_bins_debug(FarArgs a, const long lo
     const long long lin = pts[k / a.n_atoms];
     const int ix = (int)(lin % a.n1x), iy = (int)((lin / a.n1x) % a.n1y), iz = (int)(lin / ((long long)a.n1x * a.n1y));
     const int ox = ix / FRAME_X * FRAME_X, oy = iy / FRAME_Y * FRAME_Y, oz = iz / FRAME_Z * FRAME_Z;
-    const float ax = frame_atom_coord(a.ax128[at], frame_origin_bins(ox, a.nex, a.spacing_adiv));
-    const float ay = frame_atom_coord(a.ay128[at], frame_origin_bins(oy, a.ney, a.spacing_adiv));
-    const float az = frame_atom_coord(a.az128[at], frame_origin_bins(oz, a.nez, a.spacing_adiv));
-    const float s = far_pair_s(ay, az, frame_point_coord(iy - oy, a.spacing_adiv),
-                               frame_point_coord(iz - oz, a.spacing_adiv));
-    const float t = fminf(far_pair_t(ax, frame_point_coord(ix - ox, a.spacing_adiv), s), FAR_CLAMP_T);
+    const float ax = frame_atom_coord(a.ax128[at], frame_origin_bins(ox + FRAME_X / 2, a.nex, a.spacing_adiv));
+    const float ay = frame_atom_coord(a.ay128[at], frame_origin_bins(oy + FRAME_Y / 2, a.ney, a.spacing_adiv));
+    const float az = frame_atom_coord(a.az128[at], frame_origin_bins(oz + FRAME_Z / 2, a.nez, a.spacing_adiv));
+    const float s = far_pair_s(ay, az, frame_point_coord(iy - oy - FRAME_Y / 2, a.spacing_adiv),
+                               frame_point_coord(iz - oz - FRAME_Z / 2, a.spacing_adiv));
+    const float t = fminf(far_pair_t(ax, frame_point_coord(ix - ox - FRAME_X / 2, a.spacing_adiv), s), FAR_CLAMP_T);
     const int kl = (int)(__float_as_uint(__fmaf_rz(t, a.edge_lo, 8388608.f)) - MAGIC_BITS);
     const int kh = (int)(__float_as_uint(__fmaf_rz(t, a.edge_hi, 8388608.f)) - MAGIC_BITS);
     fp32[k] = (int)(__float_as_uint(__fadd_rz(t, 8388608.f)) - MAGIC_BITS);

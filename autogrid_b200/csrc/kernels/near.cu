@@ -47,8 +47,8 @@ __global__ void __launch_bounds__(NB_THREADS, 2) k_near_exact(DevProblem p_, Nea
     const bool valid = ix < p.n1x && iy < p.n1y && iz < p.n1z;
     const long long lin = ((long long)iz * p.n1y + iy) * p.n1x + ix;
     const double sp128 = p.spacing * AG_A_DIV;
-    const int ox = ((bx * BX) / FRAME_X) * FRAME_X, oy = ((by * BY) / FRAME_Y) * FRAME_Y,
-              oz = ((bz * BZ) / FRAME_Z) * FRAME_Z;
+    const int ox = ((bx * BX) / FRAME_X) * FRAME_X + FRAME_X / 2, oy = ((by * BY) / FRAME_Y) * FRAME_Y + FRAME_Y / 2,
+              oz = ((bz * BZ) / FRAME_Z) * FRAME_Z + FRAME_Z / 2;
     const double X0 = frame_origin_bins(ox, p.nex, sp128), Y0 = frame_origin_bins(oy, p.ney, sp128),
                  Z0 = frame_origin_bins(oz, p.nez, sp128);
     const float PX = frame_point_coord(ix - ox, sp128), PY = frame_point_coord(iy - oy, sp128),

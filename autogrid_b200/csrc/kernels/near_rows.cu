@@ -65,7 +65,7 @@ struct RowsNearSmem {
     int ch[NR_THREADS];
     int seg_start[NR_SEGS], seg_off[NR_SEGS + 1];
     int total, nh;
-    // the brick: its box (A), the far frame's first point and origin (bins),
+    // the brick: its box (A), the far frame's middle point and its place (bins),
     // and the range of cells in reach.  Here and not in registers, because
     // the staging needs them again when the candidates take several chunks.
     double lo[3], hi[3], org[3];
@@ -234,7 +234,7 @@ __device__ __forceinline__ void near_rows_unit(const DevProblem &p, const NearGr
         const int n1 = tid == 0 ? p.n1x : tid == 1 ? p.n1y : p.n1z, ne = tid == 0 ? p.nex : tid == 1 ? p.ney : p.nez;
         const int first = tid == 0 ? bx * BX : tid == 1 ? by * BY : bz * BZ, step = tid == 0 ? BX : tid == 1 ? BY : BZ;
         const int fr = tid == 0 ? FRAME_X : tid == 1 ? FRAME_Y : FRAME_Z, nc = tid == 0 ? p.ncx : tid == 1 ? p.ncy : p.ncz;
-        const int o = first / fr * fr;
+        const int o = first / fr * fr + fr / 2;
         const double lo = (double)(first - ne) * p.spacing, hi = (double)(min(first + step, n1) - 1 - ne) * p.spacing;
         S.lo[tid] = lo;
         S.hi[tid] = hi;
