@@ -52,6 +52,20 @@ def test_e_map_against_oracle(tmp_path, gpu_ctx, npts, n_atoms, mode):
     plan.close()
 
 
+@pytest.mark.parametrize("n_atoms", [31, 97, 1030])
+@pytest.mark.parametrize("npts", [(8, 2, 8), (34, 10, 10), (10, 4, 12), (4, 12, 18)])
+def test_e_map_of_boxes_cut_in_z(tmp_path, gpu_ctx, npts, n_atoms):
+    """Last z frames of 1, 3 and 5 planes, whose warps share the atoms out
+    among 8, 4 and 2 groups: fewer blocks of 32 atoms than groups, a rest, and
+    more than one tile."""
+    from oracle.oracle import oracle_points
+    _, prob = make_case(tmp_path, "cut", n_atoms, npts, seed=sum(npts) + n_atoms, ligand_types=["C"])
+    e = prob.scalars["elec_map"]
+    ref, flags = oracle_points(prob)
+    got = gpu_ctx.compute(prob, "fp32").reshape(prob.n_maps, -1)[e]
+    assert not ((np.abs(got - ref[e]) > _bound(prob)) & (flags == 0)).any()
+
+
 @pytest.mark.parametrize("mode", ["table", "beyond_256A", "const"])
 @pytest.mark.parametrize("npts,n_atoms", [((2, 2, 2), 3), ((14, 8, 6), 300), ((16, 6, 8), 257), ((34, 18, 4), 1100)])
 def test_fp64_e_map(tmp_path, gpu_ctx, npts, n_atoms, mode):
