@@ -4,12 +4,19 @@
 //     e(p) = sum_a q_a F(r_pa),   F(r) = T(A_DIV r) / max(r, 0.5),
 // T the table of eps factor * coeff_estat, constant past its last bin.
 // (The FP32 kernels are in diff_emap_rows.cu.)
-//   k_emap_lin      forward: one thread per point, atoms staged through shared
+//   k_emap_lin      forward: 256 points per block, atoms staged through shared
 //                   memory, the table resident in shared memory;
-//   k_emap_lin_adj  adjoint: one thread per atom, points (with dL/de) staged
+//   k_emap_lin_adj  adjoint: 256 atoms per block, points (with dL/de) staged
 //                   through shared memory,
 //                     dL/dq_a = sum_p g(p) F(r),
 //                     dL/dx_a = sum_p g(p) q_a F'(r) (x_a - x_p) / r.
+// The table takes 128 KB, so one block fits an SM; its 1,024 threads share each
+// point's (atom's) sum out among EL_SPLIT of them, which meet in shared memory.
+// With a thread for each, 8 warps per SM, the kernels waited on the chain of
+// the distance's FP64 operations: 1,000 atoms x 33^3 points forward 153 -> 74
+// us, adjoint 163 -> 97 us.
+#include <algorithm>
+
 #include "agb_device.cuh"
 #include "diff.h"
 
@@ -17,7 +24,7 @@ namespace agb {
 
 namespace {
 
-constexpr int EL_THREADS = 256, EL_TILE = 256;
+constexpr int EL_SPLIT = 4, EL_OWNERS = 256, EL_THREADS = EL_SPLIT * EL_OWNERS, EL_TILE = 1024;
 
 // Table value and slope at x = A_DIV r, and 1/r, from r^2 (FP64 reciprocal
 // square root, about 2 ulp).
@@ -43,7 +50,8 @@ __global__ void __launch_bounds__(EL_THREADS) k_emap_lin(DiffArgs a, const R2<do
     const ConfView v = conf_view(a, DiffGrads{}, blockIdx.y);  // blockIdx.y: conformer
     emap += (long long)blockIdx.y * a.n_maps_out * a.P;
 
-    const long long lin = (long long)blockIdx.x * EL_THREADS + threadIdx.x;
+    const int owner = threadIdx.x % EL_OWNERS, part = threadIdx.x / EL_OWNERS;
+    const long long lin = (long long)blockIdx.x * EL_OWNERS + owner;
     const bool valid = lin < a.P;
     const long long l = valid ? lin : 0;
     const int ix = (int)(l % a.n1x), iy = (int)((l / a.n1x) % a.n1y), iz = (int)(l / ((long long)a.n1x * a.n1y));
@@ -61,7 +69,7 @@ __global__ void __launch_bounds__(EL_THREADS) k_emap_lin(DiffArgs a, const R2<do
         __syncthreads();
         double acc = 0;
 #pragma unroll 4
-        for (int i = 0; i < na; i++) {
+        for (int i = part; i < na; i += EL_SPLIT) {
             const double4 at = s_atom[i];
             const double dx = at.x - cx, dy = at.y - cy, dz = at.z - cz;
             double T, slope, rs;
@@ -70,7 +78,13 @@ __global__ void __launch_bounds__(EL_THREADS) k_emap_lin(DiffArgs a, const R2<do
         }
         e += acc;
     }
-    if (valid) emap[lin] = e;
+    double *sum = (double *)s_atom + owner;
+    __syncthreads();
+    if (part) sum[(part - 1) * EL_OWNERS] = e;
+    __syncthreads();
+    if (part || !valid) return;
+    for (int k = 0; k < EL_SPLIT - 1; k++) e += sum[k * EL_OWNERS];
+    emap[lin] = e;
 }
 
 __global__ void __launch_bounds__(EL_THREADS)
@@ -85,7 +99,8 @@ k_emap_lin_adj(DiffArgs a, const R2<double> *__restrict__ gtab, const double *__
     const DiffGrads g = cv.g;
     g_e += (long long)blockIdx.z * a.n_maps_out * a.P;
 
-    const int at = blockIdx.x * EL_THREADS + threadIdx.x;
+    const int owner = threadIdx.x % EL_OWNERS, part = threadIdx.x / EL_OWNERS;
+    const int at = blockIdx.x * EL_OWNERS + owner;
     const bool valid = at < a.n_atoms;
     const double xa = valid ? cv.x[at] : 0, ya = valid ? cv.y[at] : 0, za = valid ? cv.z[at] : 0;
     const double qa = valid ? cv.q[at] : 0;
@@ -109,7 +124,7 @@ k_emap_lin_adj(DiffArgs a, const R2<double> *__restrict__ gtab, const double *__
         __syncthreads();
         double ax = 0, ay = 0, az = 0, aq = 0;
 #pragma unroll 4
-        for (int i = 0; i < np; i++) {
+        for (int i = part; i < np; i += EL_SPLIT) {
             const double4 pt = s_pt[i];
             const double dx = xa - pt.x, dy = ya - pt.y, dz = za - pt.z;
             double T, slope, rs;
@@ -123,7 +138,15 @@ k_emap_lin_adj(DiffArgs a, const R2<double> *__restrict__ gtab, const double *__
         }
         gx += ax; gy += ay; gz += az; gq += aq;
     }
-    if (valid) {
+    double4 *sum = s_pt + owner;
+    __syncthreads();
+    if (part) sum[(part - 1) * EL_OWNERS] = make_double4(gx, gy, gz, gq);
+    __syncthreads();
+    if (part == 0 && valid) {
+        for (int k = 0; k < EL_SPLIT - 1; k++) {
+            const double4 t = sum[k * EL_OWNERS];
+            gx += t.x; gy += t.y; gz += t.z; gq += t.w;
+        }
         atomicAdd(g.xyz + 3 * at, (double)(gx * qa));
         atomicAdd(g.xyz + 3 * at + 1, (double)(gy * qa));
         atomicAdd(g.xyz + 3 * at + 2, (double)(gz * qa));
@@ -131,6 +154,7 @@ k_emap_lin_adj(DiffArgs a, const R2<double> *__restrict__ gtab, const double *__
     }
 }
 
+static_assert((EL_SPLIT - 1) * EL_OWNERS <= EL_TILE, "the tile holds the parts' sums");
 constexpr size_t kEmapSmem = sizeof(R2<double>) * AG_NDIEL + sizeof(double4) * EL_TILE;
 
 }  // namespace
@@ -138,7 +162,7 @@ constexpr size_t kEmapSmem = sizeof(R2<double>) * AG_NDIEL + sizeof(double4) * E
 cudaError_t launch_emap_lin(const DiffArgs &a, const void *eps, double *emap, cudaStream_t s)
 {
     if (a.P == 0) return cudaSuccess;
-    const dim3 nb((unsigned)((a.P + EL_THREADS - 1) / EL_THREADS), (unsigned)a.n_conf);
+    const dim3 nb((unsigned)((a.P + EL_OWNERS - 1) / EL_OWNERS), (unsigned)a.n_conf);
     const cudaError_t e = cudaFuncSetAttribute(k_emap_lin, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kEmapSmem);
     if (e != cudaSuccess) return e;
     k_emap_lin<<<nb, EL_THREADS, kEmapSmem, s>>>(a, (const R2<double> *)eps, emap);
@@ -148,12 +172,11 @@ cudaError_t launch_emap_lin(const DiffArgs &a, const void *eps, double *emap, cu
 cudaError_t launch_emap_lin_adj(const DiffArgs &a, const void *eps, const double *g_e, DiffGrads g, cudaStream_t s)
 {
     if (a.n_atoms == 0 || a.P == 0) return cudaSuccess;
-    // about four blocks per SM over (atom blocks x point ranges)
-    const int atom_blocks = (a.n_atoms + EL_THREADS - 1) / EL_THREADS;
-    long long ranges = (4LL * current_device_sms() + atom_blocks - 1) / atom_blocks;
-    long long ppb = (a.P + ranges - 1) / ranges;
-    ppb = ((ppb + EL_TILE - 1) / EL_TILE) * EL_TILE;
-    if (ppb < EL_TILE) ppb = EL_TILE;
+    // about one block per SM over (atom blocks x point ranges x conformers): 2 and
+    // 4 load the table more often and gain nothing (3,000 atoms x 61^3 points)
+    const int atom_blocks = (a.n_atoms + EL_OWNERS - 1) / EL_OWNERS;
+    long long ranges = std::max(1LL, (long long)current_device_sms() / ((long long)atom_blocks * a.n_conf));
+    const long long ppb = std::max(((a.P + ranges - 1) / ranges + EL_SPLIT - 1) / EL_SPLIT * EL_SPLIT, 256LL);
     ranges = (a.P + ppb - 1) / ppb;
     dim3 grid((unsigned)atom_blocks, (unsigned)ranges, (unsigned)a.n_conf);
     const cudaError_t e = cudaFuncSetAttribute(k_emap_lin_adj, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kEmapSmem);

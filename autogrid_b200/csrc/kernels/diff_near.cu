@@ -318,12 +318,20 @@ cudaError_t launch_closest_h(const DiffArgs &a, int *ch, cudaStream_t s)
     return cudaGetLastError();
 }
 
+// The kernels are bound by the latency of the pair's FP64 operations at few
+// warps per SM.  Up to 8 slots with 4 min/max fit 128 registers with few
+// spills, for 2 blocks per SM (1,000 atoms x 33^3 points, 8 maps: forward
+// 300 -> 267 us, adjoint 457 -> 397; one block 1.07 ms for the whole call
+// against 0.99); with 16 slots the spills cost more than the second block
+// gives (16 maps: 1.96 ms against 1.70 with one block).
+static bool near_lin_small(const DiffArgs &a) { return a.n_slots <= 8 && a.n_mm <= 4; }
+
 cudaError_t launch_near_lin(const DiffArgs &a, const void *vdw, const void *sol, double *maps, const int *ch, int *mmarg,
                             cudaStream_t s)
 {
     if (a.P == 0 || a.n_slots == 0) return cudaSuccess;
-    k_near_lin<double, DF_MAXS, DF_MAXMM, 1><<<brick_grid(a), DF_THREADS, 0, s>>>(
-        a, (const R2<double> *)vdw, (const R2<double> *)sol, maps, ch, mmarg);
+    const auto kernel = near_lin_small(a) ? k_near_lin<double, 8, 4, 2> : k_near_lin<double, DF_MAXS, DF_MAXMM, 1>;
+    kernel<<<brick_grid(a), DF_THREADS, 0, s>>>(a, (const R2<double> *)vdw, (const R2<double> *)sol, maps, ch, mmarg);
     return cudaGetLastError();
 }
 
@@ -331,8 +339,8 @@ cudaError_t launch_near_lin_adj(const DiffArgs &a, const void *vdw, const void *
                                 const int *mmarg, DiffGrads g, cudaStream_t s)
 {
     if (a.P == 0 || a.n_slots == 0) return cudaSuccess;
-    k_near_lin_adj<double, DF_MAXS, DF_MAXMM, 1><<<brick_grid(a), DF_THREADS, 0, s>>>(
-        a, (const R2<double> *)vdw, (const R2<double> *)sol, g_maps, ch, mmarg, g);
+    const auto kernel = near_lin_small(a) ? k_near_lin_adj<double, 8, 4, 2> : k_near_lin_adj<double, DF_MAXS, DF_MAXMM, 1>;
+    kernel<<<brick_grid(a), DF_THREADS, 0, s>>>(a, (const R2<double> *)vdw, (const R2<double> *)sol, g_maps, ch, mmarg, g);
     return cudaGetLastError();
 }
 
