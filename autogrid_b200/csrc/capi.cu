@@ -702,10 +702,6 @@ ag_status build_plan(ag_plan *pl, const ag_problem *p, cudaStream_t s, bool pipe
         if (p->disorder_h && p->disorder[a] && p->rec_type[a] == p->hydrogen_type) m |= 1 << 13;
         meta[a] = m;
     }
-    std::vector<int> h_index;
-    for (int a = 0; a < N; a++)
-        if (p->hbond[a] == 1 || p->hbond[a] == 2) h_index.push_back(a);
-
     // cell list over the grid box grown by the near radius
     const double cs = AGB_CELL;
     double lo[3], hi[3];
@@ -859,7 +855,7 @@ ag_status build_plan(ag_plan *pl, const ag_problem *p, cudaStream_t s, bool pipe
 
     // uploads: the rest of the inputs in one copy
     double *dq, *dvol, *dsol, *drv, *drv2;
-    int *dtype, *dhb, *drexp, *dh, *dcs, *dca, *dcol;
+    int *dtype, *dhb, *drexp, *dcs, *dca, *dcol;
     uint8_t *ddis;
     float *dvdw = nullptr;
     late.add(p->charge, N, &dq);
@@ -871,7 +867,6 @@ ag_status build_plan(ag_plan *pl, const ag_problem *p, cudaStream_t s, bool pipe
     late.add(p->hbond, N, &dhb);
     late.add(p->rexp, N, &drexp);
     late.add(p->disorder, N, &ddis);
-    late.add(h_index.data(), h_index.size(), &dh);
     late.add(cell_start.data(), cell_start.size(), &dcs);
     late.add(cell_atoms.data(), cell_atoms.size(), &dca);
     late.add(colmap.data(), colmap.size(), &dcol);
@@ -899,7 +894,6 @@ ag_status build_plan(ag_plan *pl, const ag_problem *p, cudaStream_t s, bool pipe
 
     d.x = dx; d.y = dy; d.z = dz; d.q = dq; d.vol = dvol; d.solpar = dsol; d.rv = drv; d.rv2 = drv2;
     d.type = dtype; d.hbond = dhb; d.rexp = drexp; d.disorder = ddis;
-    d.n_h = (int)h_index.size(); d.h_index = dh;
     d.cell_start = dcs; d.cell_atoms = dca;
     d.vdw = pl->vdwT; d.sol_fn = dsolfn; d.reps = dreps; d.far_tab = pl->far_tab;
     if (!pinned || !vdwT.empty()) AGB_CK(cudaStreamSynchronize(s));  // sources are locals

@@ -190,9 +190,6 @@ struct DevProblem {
     const double *rv, *rv2;            // [3N]
     const int *type, *hbond, *rexp;
     const uint8_t *disorder;
-    // DS/D1 atoms in file order
-    int n_h;
-    const int *h_index;                // [n_h] file index
     // cell list over the near region
     int ncx, ncy, ncz;
     double cell0[3], cell_size;        // origin (centred frame), edge

@@ -122,7 +122,8 @@ __global__ void __launch_bounds__(NB_THREADS, 2) k_near_exact(DevProblem p_, Nea
             }
         }
     };
-    // ---- A: closest DS/D1 hydrogen
+    // ---- A: closest DS/D1 hydrogen.  Only pairs with a D1 atom in range use it,
+    // and such an atom is among the candidates.
     int ch = -1;
     if (need_h) {
         // the FP32 filter leaves the atoms whose distance can be the smallest;
@@ -143,15 +144,6 @@ __global__ void __launch_bounds__(NB_THREADS, 2) k_near_exact(DevProblem p_, Nea
                 if (r < rmin || (r == rmin && a < ch)) { rmin = r; ch = a; }
             }
         });
-        if (valid && !(rmin <= AG_NBC)) {  // nothing within 8 A: scan every DS/D1 atom in file order
-            rmin = 999999.;
-            ch = -1;
-            for (int k = 0; k < p.n_h; k++) {
-                const int a = p.h_index[k];
-                const double r = h_dist(p, a, cx, cy, cz);
-                if (r < rmin) { rmin = r; ch = a; }
-            }
-        }
     }
 
     // ---- B: pair terms

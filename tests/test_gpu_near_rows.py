@@ -36,3 +36,26 @@ def test_near_maps_against_oracle(tmp_path, gpu_ctx, name):
     twin = gpu_ctx.compute(prob, "fp64").reshape(prob.n_maps, -1)
     near = [m for m in range(prob.n_maps) if m != prob.scalars["elec_map"]]  # the twin's e map is another kernel's
     np.testing.assert_allclose(twin[near][:, free], ref[near][:, free], rtol=1e-9, atol=1e-9)
+
+
+@pytest.mark.parametrize("n_atoms,npts,spacing", [(60, (18, 18, 16), 1.0), (25, (30, 6, 8), 1.3)])
+def test_points_without_a_hydrogen_in_reach(tmp_path, gpu_ctx, n_atoms, npts, spacing):
+    """Boxes larger than the receptor: points with no DS/D1 atom within 8 A (the
+    reference takes one further away, which no pair in range reads), bricks with
+    such atoms for a part of their points, and bricks without any atom."""
+    from oracle.oracle import oracle_points
+    _, prob = make_case(tmp_path, "far_h", n_atoms, npts, seed=n_atoms, spacing=spacing,
+                        ligand_types=["A", "C", "HD", "N", "NA", "OA"])
+    a = prob.arrays
+    h = np.isin(a["hbond"], (1, 2))
+    ax = [(np.arange(n) - (n - 1) // 2) * spacing for n in prob.n1]
+    z, y, x = np.meshgrid(ax[2], ax[1], ax[0], indexing="ij")
+    r2 = ((a["coord"].reshape(-1, 3)[h][:, None] - np.stack([x, y, z], -1).reshape(-1, 3)) ** 2).sum(-1).min(0)
+    assert (r2 > 64).any() and (r2 < 64).any()
+    ref, flags = oracle_points(prob)
+    free = flags == 0
+    got = gpu_ctx.compute(prob, "fp32").reshape(prob.n_maps, -1)
+    assert tolerance_ok(got[:, free], ref[:, free]).all()
+    twin = gpu_ctx.compute(prob, "fp64").reshape(prob.n_maps, -1)
+    near = [m for m in range(prob.n_maps) if m != prob.scalars["elec_map"]]
+    np.testing.assert_allclose(twin[near][:, free], ref[near][:, free], rtol=1e-9, atol=1e-9)
