@@ -243,29 +243,23 @@ struct ag_context {
     size_t h_text_cap = 0;
     cudaEvent_t tev[4] = {nullptr, nullptr, nullptr, nullptr};  // measure and write passes
     BufferSet table_bufs;  // ag_tables_build
-    // pinned host image of a one-shot call's inputs (Stage)
-    char *h_stage = nullptr;
+    // host image of a one-shot call's inputs (Stage), kept so that its pages are
+    // touched once; pageable: pinned it saves 25 us of a 41^3-point call's 387
+    // and takes 2.7 ms or more once
+    std::unique_ptr<char[]> h_stage;
     size_t h_stage_cap = 0;
-    // The image with room for `bytes`, null where no memory can be pinned.
-    // s: the stream of the previous call's copies; they are done when that
-    // call has returned, unless it failed on its way.
+    // The image with room for `bytes`.  s: the stream of the previous call's
+    // copies; they are done when that call has returned, unless it failed on
+    // its way.
     cudaError_t stage(size_t bytes, cudaStream_t s, char **out)
     {
-        *out = nullptr;
         const cudaError_t e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) return e;
         if (bytes > h_stage_cap) {
-            if (h_stage) cudaFreeHost(h_stage);
-            h_stage = nullptr;
-            h_stage_cap = 0;
-            if (cudaHostAlloc((void **)&h_stage, bytes, cudaHostAllocDefault) != cudaSuccess) {
-                cudaGetLastError();
-                h_stage = nullptr;
-                return cudaSuccess;
-            }
+            h_stage.reset(new char[bytes]);
             h_stage_cap = bytes;
         }
-        *out = h_stage;
+        *out = h_stage.get();
         return cudaSuccess;
     }
     // the last run, whose statistics ag_context_stats() settles
@@ -416,7 +410,7 @@ cudaError_t upload(BufferSet *b, const char *name, const T *src, size_t n, T **d
 
 // The host image of several input arrays of a plan, sent to the device in one
 // copy: a copy for each array, 25 of them, cost 90 us of host time in a
-// 41^3-point one-shot call of 0.47 ms.  The image lies in `pinned`
+// 41^3-point one-shot call of 0.47 ms.  The image lies in `shared`
 // (room(bytes, arrays) of it), or in memory of its own.
 struct Stage {
     static constexpr size_t kAlign = 256;
@@ -425,9 +419,9 @@ struct Stage {
     size_t cap, used = 0;
     std::vector<std::pair<size_t, void **>> dst;
     static size_t room(size_t bytes, int arrays) { return (bytes + kAlign * (size_t)arrays + kAlign - 1) / kAlign * kAlign; }
-    Stage(size_t bytes, int arrays, char *pinned) : buf(pinned), cap(room(bytes, arrays))
+    Stage(size_t bytes, int arrays, char *shared) : buf(shared), cap(room(bytes, arrays))
     {
-        if (!pinned) {
+        if (!shared) {
             own.reset(new char[cap]);
             buf = own.get();
         }
@@ -538,7 +532,7 @@ ag_status build_plan(ag_plan *pl, const ag_problem *p, cudaStream_t s, bool pipe
     //
     // The kernels' tables are packed by kernels where the tables are on the
     // device already, and in one-shot calls, whose caller waits (41^3 points:
-    // 359 us against 469 with the tables packed on the host and an upload for
+    // 387 us against 469 with the tables packed on the host and an upload for
     // each array).  Plans pack them on the host: those of a batch are built
     // while the GPU is full of earlier instances' persistent blocks, and a
     // packing kernel would wait for them (24 instances one-shot: 26.9 ms
@@ -551,10 +545,10 @@ ag_status build_plan(ag_plan *pl, const ag_problem *p, cudaStream_t s, bool pipe
     const size_t late_bytes = (size_t)N * 168 + (cells + 1) * sizeof(int) + vdw_n * sizeof(float) +
                               (size_t)AG_NDIEL * 16 + 8192;
     constexpr int kEarly = 8, kLate = 32;
-    char *pinned = nullptr;  // for one-shot calls, which share the context's buffers too
-    if (!pl->own) AGB_CK(pl->ctx->stage(Stage::room(early_bytes, kEarly) + Stage::room(late_bytes, kLate), s, &pinned));
-    Stage early(early_bytes, kEarly, pinned);
-    Stage late(late_bytes, kLate, pinned ? pinned + Stage::room(early_bytes, kEarly) : nullptr);
+    char *shared = nullptr;  // for one-shot calls, which share the context's buffers too
+    if (!pl->own) AGB_CK(pl->ctx->stage(Stage::room(early_bytes, kEarly) + Stage::room(late_bytes, kLate), s, &shared));
+    Stage early(early_bytes, kEarly, shared);
+    Stage late(late_bytes, kLate, shared ? shared + Stage::room(early_bytes, kEarly) : nullptr);
     double *x128 = early.make(N, &pl->x128), *y128 = early.make(N, &pl->y128), *z128 = early.make(N, &pl->z128);
     float *qw = early.make(N, &pl->qw);
     double *dx, *dy, *dz, *dsolfn = nullptr, *deps = nullptr;
@@ -896,7 +890,7 @@ ag_status build_plan(ag_plan *pl, const ag_problem *p, cudaStream_t s, bool pipe
     d.type = dtype; d.hbond = dhb; d.rexp = drexp; d.disorder = ddis;
     d.cell_start = dcs; d.cell_atoms = dca;
     d.vdw = pl->vdwT; d.sol_fn = dsolfn; d.reps = dreps; d.far_tab = pl->far_tab;
-    if (!pinned || !vdwT.empty()) AGB_CK(cudaStreamSynchronize(s));  // sources are locals
+    if (!shared || !vdwT.empty()) AGB_CK(cudaStreamSynchronize(s));  // sources are locals
     return AG_OK;
 }
 
@@ -1507,7 +1501,6 @@ ag_status ag_context_destroy(ag_context *ctx)
     if (ctx->evn1) cudaEventDestroy(ctx->evn1);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     if (ctx->h_text) cudaFreeHost(ctx->h_text);
-    if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
     for (cudaEvent_t e : ctx->tev)
         if (e) cudaEventDestroy(e);
     delete ctx;
