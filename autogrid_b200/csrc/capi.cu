@@ -1220,7 +1220,7 @@ struct ag_batch {
     long long *d_far_begin = nullptr, *d_near_begin = nullptr;
     unsigned long long *d_counters = nullptr;  // kCounters: see its definition
     ag_tuning tune{};
-    int far_ctas_per_sm = FAR_CTAS_PER_SM, near_ctas_per_sm = 3;  // resident CTAs per SM of the persistent kernels
+    int far_ctas_per_sm = FAR_CTAS_PER_SM, near_ctas_per_sm = 2;  // resident CTAs per SM of the persistent kernels
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     ~ag_batch()

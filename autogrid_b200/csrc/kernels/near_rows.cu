@@ -9,8 +9,8 @@
 //            list per row of cells), with their canonical frame-relative FP32
 //            coordinates, ordered by receptor type (cell order within a type)
 //     A      closest DS/D1 atom per point (main.cpp:2986-3015): FP32
-//            prefilter, then FP64 with the reference's order; points with
-//            none within 8 A scan all of them (rare)
+//            prefilter, then FP64 with the reference's order, among the
+//            candidates (no pair reads one further away)
 //     B      per warp the staged atoms near its points, then the pair terms
 //   Distances come from the same canonical FP32 arithmetic as the far-field
 //   kernel.  Whenever an FP32 quantity lies within its error bound of a
@@ -23,7 +23,8 @@
 //
 // What bounds it: latency (42% of issue slots at 16 warps per SM: the directional
 // factors' dependency chains and the row gathers) and the L1 data path (59%).
-// 127^3 points x 10,000 atoms x 16 maps: 2.54 -> 1.94 ms; the gain came from
+// 127^3 points x 10,000 atoms x 16 maps: 2.54 -> 1.94 ms (1.74 without
+// the scan described at phase A); the gain came from
 // 32-byte row loads, the ambiguous pairs' FP64 code behind calls (their guard
 // now the proven error bound: 0.12% instead of 0.4% of pairs take it), the
 // brick's geometry out of the pair loop's registers, H-bond maps gathered in
