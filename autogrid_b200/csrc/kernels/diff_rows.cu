@@ -34,6 +34,7 @@
 #include "diff_pair.cuh"
 
 #include "diff_brick.cuh"
+#include "type_sort.cuh"
 #include "warp_sums.cuh"
 
 namespace agb {
@@ -66,7 +67,7 @@ template <bool ANG, bool SOL> struct RowsSmem {
     float4 rv[ANG ? DF_STAGE : 1], rv2[ANG ? DF_STAGE : 1];
     union {
         unsigned short wl[DF_WARPS][DF_STAGE];  // per warp: staged slots near its points
-        int tcnt[DF_STAGE / 32][32];            // staging by receptor type: per 32-candidate slice and type
+        int tcnt[DF_WARPS][32];                 // staging by receptor type (type_sorted_place)
     };
     float wbox[DF_WARPS][6];                    // per warp: its points' box (lo xyz, hi xyz), A
     float2 sol[SOL ? AG_NEINT : 1];
@@ -105,46 +106,18 @@ __device__ __forceinline__ void rows_box(const Brick &bk, float px, float py, fl
 }
 
 // Stage candidates [c0, c0 + DF_STAGE) of the brick, ordered by receptor type
-// by a stable counting sort (cell order within a type), so that the warps walk
-// the table of one type at a time.  Slice k (one warp's candidates) is ranked
-// by its warp; tcnt[k][t] holds the slice's count of type t, then the slot of
-// its first such candidate.  All threads call it; it ends with a barrier.
+// (cell order within a type), so that the warps walk the table of one type at
+// a time.  All threads call it; it ends with a barrier.
 template <bool ANG, bool SOL>
 __device__ __forceinline__ void rows_stage(const DiffArgs &a, const ConfView &v, RowsSmem<ANG, SOL> &sm, int c0)
 {
     static_assert(DF_STAGE == DF_THREADS, "one candidate per thread");
-    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    const int t = threadIdx.x;
     const bool in = c0 + t < sm.sg.total;
-    sm.tcnt[w][lane] = 0;
     const int ia = in ? brick_atom(v, sm.sg, c0 + t) : 0;
-    const int meta = in ? a.meta[ia] : 0, type = in ? meta & DM_TYPE_MASK : 32;  // 32: past the chunk
-    const unsigned same = __match_any_sync(0xffffffffu, type);
-    const int rank = __popc(same & ((1u << lane) - 1u));
-    if (in && rank == 0) sm.tcnt[w][type] = __popc(same);
-    __syncthreads();
-    if (w == 0) {  // lane: a type's slots, slices in order, after every lower type
-        int cnt[DF_WARPS], run = 0;
-#pragma unroll
-        for (int k = 0; k < DF_WARPS; k++) {
-            cnt[k] = sm.tcnt[k][lane];
-            run += cnt[k];
-        }
-        int first = run;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int u = __shfl_up_sync(0xffffffffu, first, o);
-            if (lane >= o) first += u;
-        }
-        first -= run;
-#pragma unroll
-        for (int k = 0; k < DF_WARPS; k++) {
-            sm.tcnt[k][lane] = first;
-            first += cnt[k];
-        }
-    }
-    __syncthreads();
+    const int meta = in ? a.meta[ia] : 0;
+    const int j = type_sorted_place<DF_WARPS>(sm.tcnt, in ? meta & DM_TYPE_MASK : 32, in);
     if (in) {
-        const int j = sm.tcnt[w][type] + rank;
         sm.pos[j] = make_float4((float)v.x[ia], (float)v.y[ia], (float)v.z[ia], __int_as_float(meta));
         sm.idx[j] = ia;
         if (SOL) {
