@@ -626,8 +626,10 @@ __device__ __forceinline__ void near_rows_unit(const DevProblem &p, const NearGr
                                 } else {
                                     if (m < NG_MM) {  // min/max maps are placed first by the host
                                         v *= fac;
-                                        S.hmin[m < NG_MM ? m : 0][tid] = fminf(S.hmin[m < NG_MM ? m : 0][tid], v);
-                                        S.hmax[m < NG_MM ? m : 0][tid] = fmaxf(S.hmax[m < NG_MM ? m : 0][tid], v);
+                                        // comparisons as the reference's: a NaN is stored
+                                        const float lo = S.hmin[m < NG_MM ? m : 0][tid], hi = S.hmax[m < NG_MM ? m : 0][tid];
+                                        S.hmin[m < NG_MM ? m : 0][tid] = lo < v ? lo : v;
+                                        S.hmax[m < NG_MM ? m : 0][tid] = hi > v ? hi : v;
                                     }
                                     continue;
                                 }
@@ -647,7 +649,8 @@ __device__ __forceinline__ void near_rows_unit(const DevProblem &p, const NearGr
         for (int m = 0; m < NGK; m++) {
             if (m >= g.ng) break;
             float v = (m & 1) ? E[m / 2].y : E[m / 2].x;
-            if (m < NG_MM && S.hmin[m < NG_MM ? m : 0][tid] <= S.hmax[m < NG_MM ? m : 0][tid])  // some pair entered
+            // some pair entered (also where it left a NaN): until then min > max
+            if (m < NG_MM && !(S.hmin[m < NG_MM ? m : 0][tid] > S.hmax[m < NG_MM ? m : 0][tid]))
                 v += S.hmin[m < NG_MM ? m : 0][tid] + fmaxf(S.hmax[m < NG_MM ? m : 0][tid], 0.f);
             v += (float)g.sp[m] * D1 + (float)g.vp[m] * D2;
             const size_t o = (size_t)g.out_map[m] * (size_t)p.P + (size_t)lin;
