@@ -76,11 +76,15 @@ __device__ __forceinline__ ErPoints er_points(const DiffArgs &a, int f)
     p.iy = f / nfx % nfy * FRAME_Y + ty;
     p.iz = oz + tz;
     p.warp_in = oz + 2 * v < a.n1z;
+    // a point of the frame past the box takes the coordinates of the box's last:
+    // the distances are then those of points in the box, and its weight of 0
+    // meets no table value (which may be no number) that these do not
+    const int lx = a.n1x - 1 - (p.ix - tx), ly = a.n1y - 1 - (p.iy - ty), lz = a.n1z - 1 - oz;
 #pragma unroll
     for (int j = 0; j < ER_PAIRS; j++)
-        p.npx[j] = make_float2(-frame_point_coord(tx + 8 * j, bin), -frame_point_coord(tx + 8 * j + 4, bin));
-    p.npy = make_float2(-frame_point_coord(ty, bin), -frame_point_coord(ty + 4, bin));
-    p.npz = -frame_point_coord(tz, bin);
+        p.npx[j] = make_float2(-frame_point_coord(min(tx + 8 * j, lx), bin), -frame_point_coord(min(tx + 8 * j + 4, lx), bin));
+    p.npy = make_float2(-frame_point_coord(min(ty, ly), bin), -frame_point_coord(min(ty + 4, ly), bin));
+    p.npz = -frame_point_coord(min(tz, lz), bin);
     return p;
 }
 

@@ -43,3 +43,30 @@ def test_minmax_maps_keep_what_is_not_finite(tmp_path, gpu_ctx, ligand, classes,
         np.testing.assert_array_equal(got[m][hit], twin[m][hit].astype(np.float32))
         assert tolerance_ok(got[m][~hit], twin[m][~hit]).all()
         np.testing.assert_array_equal(np.delete(got, m, 0), np.delete(finite, m, 0))
+
+
+def test_gradient_with_a_dielectric_beyond_every_pair(tmp_path, gpu_ctx):
+    """Dielectric values at distances that no atom and point have do not reach
+    the gradient (the kernels pad the box to whole frames)."""
+    from autogrid_b200 import Diff
+    _, prob = make_case(tmp_path, "far_eps", 200, (4, 6, 2), seed=3, ligand_types=["C", "OA"])
+    n1, ne, sp = prob.n1, prob.ne, prob.scalars["spacing"]
+    c = prob.arrays["coord"].reshape(-1, 3)
+    lo, hi = -np.array(ne) * sp, (np.array(n1) - 1 - np.array(ne)) * sp
+    reach = np.sqrt((np.maximum(abs(c - lo), abs(c - hi)) ** 2).sum(1).max())
+    w = np.zeros(prob.map_shape, np.float32)
+    w[prob.scalars["elec_map"]] = np.random.default_rng(1).normal(size=prob.map_shape[1:])
+    assert prob.scalars["dddiel"]
+    grads = []
+    for value in (None, np.nan, np.inf):
+        if value is not None:
+            prob.arrays["r_epsilon_fn"][int(reach * 128) + 4:] = value
+        d = Diff(gpu_ctx, prob, "fp32")
+        d.forward()
+        grads.append((d.maps(), d.backward(w)))
+        d.close()
+    for maps, g in grads[1:]:
+        np.testing.assert_array_equal(maps, grads[0][0])
+        for key in ("coord", "charge"):
+            norm = np.linalg.norm(grads[0][1][key])
+            assert np.linalg.norm(g[key] - grads[0][1][key]) <= 1e-6 * norm, key
