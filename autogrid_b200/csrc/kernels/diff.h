@@ -89,6 +89,7 @@ struct DiffArgs {
     // an H-bond action
     const float *row_v, *row_d;
     int row_stride, n_hb;
+    int rows_finite;             // 1: every entry of the rows is a finite number
     unsigned cls_plain;
     unsigned long long cls_act[16];
     double cov_pos[3], cov_half_width, cov_barrier;
