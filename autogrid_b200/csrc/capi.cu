@@ -629,7 +629,8 @@ ag_status build_plan(ag_plan *pl, const ag_problem *p, cudaStream_t s, bool pipe
     }
     void *v = nullptr;
     const size_t P = (size_t)d.P;
-    if (pl->n_chunks > 0 && pl->opts.precision != AG_PREC_FP64) {
+    // (a batch sizes the sums and the edge bits of its plans itself, for its own chunks)
+    if (pl->n_chunks > 0 && pl->opts.precision != AG_PREC_FP64 && !B->arena) {
         AGB_CK(B->ensure("far_partial", (size_t)pl->n_chunks * P * sizeof(float), &v));
         pl->far_partial = (float *)v;
     } else {
@@ -1220,6 +1221,7 @@ struct ag_batch {
     long long *d_far_begin = nullptr, *d_near_begin = nullptr;
     unsigned long long *d_counters = nullptr;  // kCounters: see its definition
     ag_tuning tune{};
+    int far_chunking = 0;  // far_chunk_atoms
     int far_ctas_per_sm = FAR_CTAS_PER_SM, near_ctas_per_sm = 2;  // resident CTAs per SM of the persistent kernels
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -1236,15 +1238,44 @@ namespace {
 long long far_units(const FarArgs &a) { return (long long)a.nfx * a.nfy * a.nfz * ((a.n_atoms + a.chunk_atoms - 1) / std::max(1, a.chunk_atoms)); }
 
 // Atoms per far-field unit of an instance: all, or chunks of 2048 or 512.
-constexpr int kFarChunkings = 3;
 int far_chunk_atoms(int chunking, int n_atoms)
 {
     const int all = std::max(n_atoms, 1);
     return chunking == 0 ? all : std::min(all, chunking == 1 ? 2048 : 512);
 }
 
+// Waves of far units that a batch's instances make.
+double batch_far_waves(const ag_batch *b, int chunking)
+{
+    long long units = 0;
+    for (const auto &pl : b->plans) {
+        const DevProblem &d = pl->dp;
+        if (d.elec_map < 0 || d.n_atoms == 0) continue;
+        const int c = far_chunk_atoms(chunking, d.n_atoms);
+        units += (long long)frames_x(d.n1x) * frames_y(d.n1y) * frames_z(d.n1z) * ((d.n_atoms + c - 1) / c);
+    }
+    return (double)units / (b->ctx->sms * FAR_CTAS_PER_SM);
+}
+
+// The finest chunking a batch may take, and the one it takes untuned.  Smaller
+// units fill the last wave, which counts where waves are few, and load the
+// table more often.  Run of ensembles of 1,000-12,000 atoms and 21^3-101^3
+// points (waves of whole instances and of 2048-atom units; then ms with whole
+// instances, 2048 and 512 atoms):
+//    2 boxes   1.0   1.6    1.68   0.85   0.82
+//    3         1.3   2.6    1.97   1.93   1.93
+//    6         2.7   7.1    3.82   3.69   3.76
+//   12         5.6  22.6    9.84   9.73   9.99
+//   24        14.0  33.0   17.03  17.07  17.52
+//   48        31.4  83.3   39.94  40.04  41.13
+// The partial sums grow with the units (8 KB each): the line at 6 waves also
+// keeps those of 512-atom units below 60 MB per batch.
+int batch_finest_chunking(const ag_batch *b) { return batch_far_waves(b, 1) < 6.0 ? 2 : 1; }
+int batch_default_chunking(const ag_batch *b) { return batch_far_waves(b, 0) >= 10.0 ? 0 : batch_finest_chunking(b); }
+
 ag_status batch_upload_far(ag_batch *b, int chunking)
 {
+    b->far_chunking = chunking;
     b->far_begin.assign(1, 0);
     for (size_t i = 0; i < b->far.size(); i++) {
         FarArgs &a = b->far[i];
@@ -1351,8 +1382,8 @@ ag_status batch_autotune(ag_batch *b)
     t = ag_tuning{};
     double best_far = 1e30, best_near = 1e30;
     int best_tile = 512, best_chunked = 0, best_shape = 0;
-    const int tiles[2] = {512, 1024};
-    for (int chunked = 0; chunked < kFarChunkings; chunked++) {
+    const int tiles[2] = {512, 1024}, finest = batch_finest_chunking(b);
+    for (int chunked = 0; chunked <= finest; chunked++) {
         ag_status st = batch_upload_far(b, chunked);
         if (st != AG_OK) return st;
         for (int ti = 0; ti < 2; ti++) {
@@ -1376,7 +1407,7 @@ ag_status batch_autotune(ag_batch *b)
         if (n < best_near) { best_near = n; best_shape = shape; }
     }
     t.far_tile = best_tile;
-    t.far_chunked = best_chunked;
+    t.far_chunked = best_chunked != 0;
     t.near_shape = best_shape;
     t.far_ms = best_far;
     t.near_ms = best_near;
@@ -1945,11 +1976,12 @@ static ag_status batch_create(ag_context *ctx, const ag_problem *const *problems
     });
     b->near_begin.assign(1, 0);
     b->red_begin.assign(1, 0);
+    const int finest = batch_finest_chunking(b.get());
     for (int i : order) {
         ag_plan *pl = b->plans[i].get();
-        // each instance's buffers must hold every chunking of batch_upload_far
+        // each instance's buffers must hold every chunking that the batch may take
         int max_chunks = 1;
-        for (int k = 0; k < kFarChunkings; k++) {
+        for (int k = 0; k <= finest; k++) {
             const int c = far_chunk_atoms(k, pl->dp.n_atoms);
             max_chunks = std::max(max_chunks, (pl->dp.n_atoms + c - 1) / c);
         }
@@ -1960,7 +1992,7 @@ static ag_status batch_create(ag_context *ctx, const ag_problem *const *problems
             if (pl->far_mode != FAR_TAB_CONST) {
                 const int nframes = frames_x(pl->dp.n1x) * frames_y(pl->dp.n1y) * frames_z(pl->dp.n1z);
                 size_t eb = 0;
-                for (int k = 0; k < kFarChunkings; k++) {
+                for (int k = 0; k <= finest; k++) {
                     const int c = far_chunk_atoms(k, pl->dp.n_atoms);
                     eb = std::max(eb, far_edge_bits_bytes((pl->dp.n_atoms + c - 1) / c, c, nframes));
                 }
@@ -2017,13 +2049,10 @@ static ag_status batch_create(ag_context *ctx, const ag_problem *const *problems
         if (st != AG_OK) return st;
     } else {
         b->tune = ag_tuning{};
-        // 24 boxes of 1,000-12,000 atoms in one call: 512-atom chunks 23.6 ms,
-        // 2048 23.7 ms, whole instances 26.2 ms (the last units of a group of
-        // few boxes leave the GPU idle)
-        b->tune.far_chunked = 2;
-        st = batch_upload_far(b.get(), b->tune.far_chunked);
+        st = batch_upload_far(b.get(), batch_default_chunking(b.get()));
         if (st != AG_OK) return st;
         b->tune.far_tile = 512;
+        b->tune.far_chunked = b->far_chunking != 0;
         b->tune.near_shape = 0;
     }
     // final near unit table for the chosen shape

@@ -352,7 +352,7 @@ ag_status ag_emap_compute_noalloc(int32_t device, int32_t n_atoms, const double 
 typedef struct ag_batch ag_batch;
 typedef struct ag_tuning {
     int32_t far_tile;         /* atoms per shared-memory tile (512, 1024)          */
-    int32_t far_chunked;      /* atoms per unit: 0 all, 1 up to 2048, 2 up to 512  */
+    int32_t far_chunked;      /* 1: atoms split in chunks per unit                 */
     int32_t near_shape;       /* 0: 8x8x4, 1: 8x4x8, 2: 4x8x8 points per brick     */
     int32_t candidates;       /* configurations timed                             */
     double  far_ms, near_ms;  /* device time of the chosen far / near launches    */
