@@ -470,12 +470,12 @@ ag_status ag_diff_create_batch(ag_context *ctx, const ag_problem *p, const ag_op
         // values, then steps; a type's last value row is there twice
         const size_t n32 = n_rows / AG_NEINT * DF_ROWS;
         std::vector<float> rows(2 * n32 * A.row_stride, 0.f);
-        A.rows_finite = 1;
+        A.weigh_all = std::all_of(slots.begin(), slots.end(), [](const Slot &sl) { return sl.tab >= 0 || sl.kind == DK_D || sl.desolv; });
         each_vdw(p, A, [&](size_t row, int s, double v, double dv) {
             const size_t t = row / AG_NEINT, b = row % AG_NEINT, o = (t * DF_ROWS + b) * A.row_stride + s;
             rows[o] = (float)v;
             rows[n32 * A.row_stride + o] = (float)dv;
-            if (!std::isfinite((float)v) || !std::isfinite((float)dv)) A.rows_finite = 0;
+            if (!std::isfinite((float)v) || !std::isfinite((float)dv)) A.weigh_all = 0;
             if (b == AG_NEINT - 1) rows[o + A.row_stride] = (float)v;
         });
         std::vector<R2<float>> sol, eps;

@@ -89,7 +89,8 @@ struct DiffArgs {
     // an H-bond action
     const float *row_v, *row_d;
     int row_stride, n_hb;
-    int rows_finite;             // 1: every entry of the rows is a finite number
+    int weigh_all;               // 1: the adjoint may multiply every slot's weight with its row: all entries
+                                 // are finite, and every slot has a pair or desolvation term
     unsigned cls_plain;
     unsigned long long cls_act[16];
     double cov_pos[3], cov_half_width, cov_barrier;

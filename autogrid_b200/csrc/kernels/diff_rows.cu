@@ -339,8 +339,8 @@ k_rows(DiffArgs a, const float2 *__restrict__ sol, float *__restrict__ maps, con
 }
 
 // A slot of weight 0 adds nothing, also where its table entry is no number: the
-// entries of such slots become 0.  Rows of finite numbers need none of it
-// (FINITE; a test at run time took 8 us of the 2.13 ms step of 4,000 atoms).
+// entries of such slots become 0.  Most map sets need none of it (ALL,
+// DiffArgs::weigh_all; a test at run time took 8 us of the 2.13 ms step of 4,000 atoms).
 template <int NB>
 __device__ __forceinline__ void drop_unweighted(const float2 (&gs)[4 * NB], Row8 &r, int k8)
 {
@@ -353,7 +353,7 @@ __device__ __forceinline__ void drop_unweighted(const float2 (&gs)[4 * NB], Row8
 
 // Adjoint of one in-range pair of a class whose slots are all plain:
 // dL/d(atom position) and, with desolvation, dL/dq.
-template <int NB, bool SOL, bool FINITE>
+template <int NB, bool SOL, bool ALL>
 __device__ __forceinline__ void plain_adjoint(const DiffArgs &a, const RowGeom &g, unsigned ro, const float2 *sol,
                                               const float4 *aux, const float2 (&gs)[4 * NB], float gD1, float gD2,
                                               float *out)
@@ -365,7 +365,7 @@ __device__ __forceinline__ void plain_adjoint(const DiffArgs &a, const RowGeom &
     for (int k8 = 0; k8 < NB; k8++)
         if (8 * k8 < a.n_slots) {
             rd8[k8] = load_row8(a.row_d + ro + 8 * k8);
-            if (!FINITE) drop_unweighted<NB>(gs, rd8[k8], k8);
+            if (!ALL) drop_unweighted<NB>(gs, rd8[k8], k8);
         }
     if (SOL) {
         const float2 t = sol[g.b];
@@ -388,7 +388,7 @@ __device__ __forceinline__ void plain_adjoint(const DiffArgs &a, const RowGeom &
         for (int k8 = 0; k8 < NB; k8++)
             if (8 * k8 < a.n_slots) {
                 Row8 r = load_row8(a.row_v + ro + 8 * k8);
-                if (!FINITE) drop_unweighted<NB>(gs, r, k8);
+                if (!ALL) drop_unweighted<NB>(gs, r, k8);
 #pragma unroll
                 for (int i = 0; i < 4; i++) S = __ffma2_rn(gs[4 * k8 + i], __ffma2_rn(f2, rd8[k8].p[i], r.p[i]), S);
             }
@@ -400,7 +400,7 @@ __device__ __forceinline__ void plain_adjoint(const DiffArgs &a, const RowGeom &
     out[2] = gx * g.d[2];
 }
 
-template <int MS, int MM, int MINB, bool ANG, bool SOL, bool FINITE>
+template <int MS, int MM, int MINB, bool ANG, bool SOL, bool ALL>
 __global__ void __launch_bounds__(DF_THREADS, MINB)
 k_rows_adj(DiffArgs a, const float2 *__restrict__ sol, const float *__restrict__ g_maps, const int *__restrict__ chs,
            const int *__restrict__ mmarg, DiffGrads gr_all)
@@ -437,7 +437,7 @@ k_rows_adj(DiffArgs a, const float2 *__restrict__ sol, const float *__restrict__
                     gD2 = fmaf(w, (float)a.slot_vp[s], gD2);
                 }
             }
-            if (a.slot_tab[s] < 0) w = 0.f;  // no pair term: the weight goes nowhere else
+            if (!ALL && a.slot_tab[s] < 0) w = 0.f;  // no pair term: the weight goes nowhere else
         }
         if (s & 1) gs[s >> 1].y = w;
         else gs[s >> 1].x = w;
@@ -470,7 +470,7 @@ k_rows_adj(DiffArgs a, const float2 *__restrict__ sol, const float *__restrict__
                     RowGeom g;
                     if (!rows_geom(A, px, py, pz, g) || !bk.valid || k + u >= cnt) continue;
                     const unsigned ro = (unsigned)((__float_as_int(A.w) & DM_TYPE_MASK) * DF_ROWS + g.b) * (unsigned)a.row_stride;
-                    plain_adjoint<NB, SOL, FINITE>(a, g, ro, sm.sol, sm.aux + (SOL ? j : 0), gs, gD1, gD2, out + 4 * u);
+                    plain_adjoint<NB, SOL, ALL>(a, g, ro, sm.sol, sm.aux + (SOL ? j : 0), gs, gD1, gD2, out + 4 * u);
                 }
                 const float sum = warp_sums(out, lane);
                 const int n = (lane >> 2) & 3, u = lane >> 4;
@@ -495,7 +495,7 @@ k_rows_adj(DiffArgs a, const float2 *__restrict__ sol, const float *__restrict__
             const unsigned ro = (unsigned)((meta & DM_TYPE_MASK) * DF_ROWS + g.b) * (unsigned)a.row_stride;
             if (in) {
                 if (plain) {
-                    plain_adjoint<NB, SOL, FINITE>(a, g, ro, sm.sol, sm.aux + (SOL ? j : 0), gs, gD1, gD2, out);
+                    plain_adjoint<NB, SOL, ALL>(a, g, ro, sm.sol, sm.aux + (SOL ? j : 0), gs, gD1, gD2, out);
                 } else {
                     const float dw = (float)AG_NEINT - g.x < 1.f ? -1.f : 0.f;
                     const float dn[3] = {g.d[0] * g.inv, g.d[1] * g.inv, g.d[2] * g.inv};
@@ -506,7 +506,7 @@ k_rows_adj(DiffArgs a, const float2 *__restrict__ sol, const float *__restrict__
                         if (8 * k8 < a.n_slots) {
                             rd8[k8] = load_row8(a.row_d + ro + 8 * k8);
                             rv8[k8] = load_row8(a.row_v + ro + 8 * k8);
-                            if (!FINITE) {
+                            if (!ALL) {
                                 drop_unweighted<NB>(gs, rd8[k8], k8);
                                 drop_unweighted<NB>(gs, rv8[k8], k8);
                             }
@@ -591,7 +591,7 @@ k_rows_adj(DiffArgs a, const float2 *__restrict__ sol, const float *__restrict__
 
 // The instantiation of a map set: 8 or 16 slots; no, at most 2 or at most 8
 // min/max slots; directional factors or not; desolvation terms or not; the
-// adjoint for rows of finite numbers or any.
+// adjoint for map sets with weigh_all or any.
 // <MS, MM, blocks per SM>: the Vina maps measured the same with 3 and 4 blocks
 // and 3-5% slower with 5 and 6 (the registers spill); the 8-slot AD4 forward
 // the same with 2 and 3, its adjoint 10% faster with 2 (it spills with 3).
@@ -622,7 +622,7 @@ cudaError_t launch_rows_adj(const DiffArgs &a, const void *sol, const float *g_m
                             DiffGrads g, cudaStream_t s)
 {
     if (a.P == 0 || a.n_slots == 0) return cudaSuccess;
-    if (a.rows_finite) ROWS_LAUNCH(ADJOINT, 2, a, (const float2 *)sol, g_maps, ch, mmarg, g);
+    if (a.weigh_all) ROWS_LAUNCH(ADJOINT, 2, a, (const float2 *)sol, g_maps, ch, mmarg, g);
     else ROWS_LAUNCH(ADJOINT_ANY, 2, a, (const float2 *)sol, g_maps, ch, mmarg, g);
     return cudaGetLastError();
 }
