@@ -155,6 +155,8 @@ SIGNATURES = {
     # measurement and test helpers (include/autogrid_b200_diag.h)
     "ag_diag_peak_rates": (C.c_int, [C.c_int32, C.POINTER(C.c_double), C.POINTER(C.c_double),
                                      C.POINTER(C.c_double)]),
+    "ag_diag_far_units": (C.c_int, [C.c_int32, C.c_int32, C.c_int32, C.c_float, C.c_float, C.POINTER(C.c_int64)]),
+    "ag_diag_root_errors": (C.c_int, [C.c_int32, C.POINTER(C.c_int64), C.c_int32, C.c_int32, C.POINTER(C.c_double)]),
     "ag_diag_rsqrt_error": (C.c_int, [C.c_int32, C.c_int32, C.c_int32, C.POINTER(C.c_double)]),
     "ag_diag_far_bins": (C.c_int, [C.c_void_p, C.POINTER(ag_problem), C.c_int32, C.c_void_p, C.c_void_p,
                                    C.c_void_p, C.c_void_p]),

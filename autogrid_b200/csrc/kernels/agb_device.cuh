@@ -78,6 +78,39 @@ __device__ __forceinline__ double rsqrt_f64(double x)
     return __fma_rn(__dmul_rn(y, e), __fma_rn(0.375, e, 0.5), y);
 }
 
+// sqrt(x) and, in `inv`, the approximation of 1/sqrt(x) that it shares:
+// Markstein's correction of x * inv, correctly rounded for every float in
+// [1e-12, 64] (ag_diag_root_errors).
+__device__ __forceinline__ float sqrt_markstein(float x, float &inv)
+{
+    inv = rsqrt_approx(x);
+    const float r1 = __fmul_rn(x, inv);
+    return __fmaf_rn(__fmaf_rn(-r1, r1, x), 0.5f * inv, r1);
+}
+
+// The far kernel works in units of 2^24 bins: a distance is then t * 2^-24, and
+// the product with edge * 2^-125, rounded toward zero into the subnormal
+// range, is the integer floor(t * edge) in the low bits of the float.
+// Scaling by powers of two is exact and rsqrt.approx repeats its mantissas
+// every two binades (ag_diag_far_units), so every t equals the near kernel's
+// and the fix-up's.
+constexpr float FAR_DOWN = 5.9604644775390625e-08f;          // 2^-24
+constexpr float FAR_TINY_T2 = TINY_T2 * FAR_DOWN * FAR_DOWN;
+constexpr float FAR_EDGE_DOWN = 2.3509887016445750e-38f;     // 2^-125
+// -floor(t * edge_lo) of a packed pair of distances in those units (nlom:
+// -edge_lo * FAR_EDGE_DOWN), and n + floor(t * edge_hi) (him: edge_hi * FAR_EDGE_DOWN).
+__device__ __forceinline__ float2 far_units_lo(float2 t, float2 nlom) { return __fmul2_rz(t, nlom); }
+__device__ __forceinline__ float2 far_units_hi(float2 t, float2 him, float2 n) { return __ffma2_rz(t, him, n); }
+// The guard bins of a packed pair of distances in bins: bit patterns MAGIC_BITS +
+// floor(t*edge_lo) and MAGIC_BITS + floor(t*edge_hi) (one FMA each, rounded
+// toward zero onto 2^23).
+__device__ __forceinline__ void far_guard_bins(float2 t, float2 lom, float2 him, float2 &lo, float2 &hi)
+{
+    const float2 magic = make_float2(8388608.f, 8388608.f);
+    lo = __ffma2_rz(t, lom, magic);
+    hi = __ffma2_rz(t, him, magic);
+}
+
 // The far kernel's distance (in bins) of a pair, from frame-relative FP32
 // inputs.  Written with explicit round-to-nearest intrinsics so no contraction
 // or reassociation can make two call sites differ.

@@ -172,15 +172,9 @@ __device__ __forceinline__ bool rows_geom(const float4 &A, float px, float py, f
     g.d[2] = A.z - pz;
     // r picks the table bin, where the slopes jump: its rounding is pinned, so
     // that forward and adjoint (and later builds) take the same bins
-    float r2 = __fmaf_rn(g.d[2], g.d[2], __fmaf_rn(g.d[1], g.d[1], __fmul_rn(g.d[0], g.d[0])));
+    const float r2 = __fmaf_rn(g.d[2], g.d[2], __fmaf_rn(g.d[1], g.d[1], __fmul_rn(g.d[0], g.d[0])));
     if (r2 > (float)(AG_NBC * AG_NBC)) return false;
-    // r = sqrt(r2), at least 1e-6 A, by Markstein's correction of r2 * (1/sqrt(r2)),
-    // which shares the approximation with 1/r; correctly rounded for every
-    // float in [1e-13, 65] (all of them compared with sqrtf)
-    r2 = fmaxf(r2, 1.0e-12f);
-    g.inv = rsqrt_approx(r2);
-    const float r1 = __fmul_rn(r2, g.inv);
-    const float r = __fmaf_rn(__fmaf_rn(-r1, r1, r2), 0.5f * g.inv, r1);
+    const float r = sqrt_markstein(fmaxf(r2, 1.0e-12f), g.inv);  // at least 1e-6 A
     g.x = r * (float)AG_A_DIV;
     g.b = min((int)g.x, AG_NEINT - 1);
     g.fx = g.x - (float)g.b;

@@ -73,16 +73,6 @@ __device__ __forceinline__ int far_exact_bin(const double *ax128, const double *
     return (int)__dmul_rn(r, (double)AG_A_DIV) | FAR_TIE_FLAG;
 }
 
-// The guard bins of a packed pair of distances: bit patterns MAGIC_BITS +
-// floor(t*edge_lo) and MAGIC_BITS + floor(t*edge_hi) (one FMA each, rounded
-// toward zero onto 2^23).
-__device__ __forceinline__ void far_guard_bins(float2 t, float2 lom, float2 him, float2 &lo, float2 &hi)
-{
-    const float2 magic = make_float2(8388608.f, 8388608.f);
-    lo = __ffma2_rz(t, lom, magic);
-    hi = __ffma2_rz(t, him, magic);
-}
-
 // A thread's place in a far-field unit: the compact 4x4x2 lane footprint per
 // warp (fewest table bank conflicts); each thread holds 8 points of one
 // x-row, x = tx + 8j and tx + 8j + 4 (j < EF_PAIRS).
@@ -108,15 +98,7 @@ __device__ __forceinline__ size_t far_bits_base(const FarArgs &a, int f, int chu
     return ((size_t)chunk * (size_t)(a.nfx * a.nfy * a.nfz) + (size_t)f) * (size_t)a.edge_words * EF_THREADS;
 }
 
-// The far kernel works in units of 2^24 bins: a distance is then t * 2^-24, and
-// the product with edge * 2^-125, rounded toward zero into the subnormal
-// range, is the integer floor(t * edge) in the low bits of the float.
-// Scaling by powers of two is exact and rsqrt.approx repeats its mantissas
-// every two binades, so every t equals the near kernel's and the fix-up's.
-constexpr float FAR_DOWN = 5.9604644775390625e-08f;          // 2^-24
-constexpr float FAR_TINY_T2 = TINY_T2 * FAR_DOWN * FAR_DOWN;
-constexpr float FAR_EDGE_DOWN = 2.3509887016445750e-38f;     // 2^-125
-constexpr int EF_GROUP = EF_THREADS / 2;                     // threads that hold a frame's points
+constexpr int EF_GROUP = EF_THREADS / 2;  // threads that hold a frame's points
 
 // Plane pairs of a frame's 4 that the box reaches, 3 counted as 4: the CTA's
 // 8 warps divide evenly among 1, 2 or 4.
@@ -238,8 +220,8 @@ __device__ __forceinline__ void far_unit_n(const FarArgs &a, int f, int chunk, c
                             continue;
                         }
                         if (CLAMP) t = make_float2(fminf(t.x, FAR_CLAMP_T * FAR_DOWN), fminf(t.y, FAR_CLAMP_T * FAR_DOWN));
-                        const float2 nlo = __fmul2_rz(t, nlom);
-                        E[r] = __ffma2_rz(t, him, j ? __fadd2_rn(E[r], nlo) : nlo);
+                        const float2 nlo = far_units_lo(t, nlom);
+                        E[r] = far_units_hi(t, him, j ? __fadd2_rn(E[r], nlo) : nlo);
                         // the sign bit leaves with the shift
                         const float T0 = lds_f32(tab_base + (__float_as_uint(nlo.x) << 2));
                         const float T1 = lds_f32(tab_base + (__float_as_uint(nlo.y) << 2));
