@@ -432,7 +432,6 @@ ag_status ag_diff_create_batch(ag_context *ctx, const ag_problem *p, const ag_op
         A.slot_map[s] = sl.map;
         A.slot_kind[s] = sl.kind;
         A.slot_tab[s] = sl.tab;
-        A.slot_mm[s] = sl.mm ? s : -1;
         A.slot_desolv[s] = sl.desolv;
         A.slot_sp[s] = (sl.kind != DK_D) ? p->map_solpar_probe[sl.map] : 0.0;
         A.slot_vp[s] = (sl.kind != DK_D) ? p->map_vol_probe[sl.map] : 0.0;

@@ -20,7 +20,6 @@ constexpr int FRAME_X = 32, FRAME_Y = 8, FRAME_Z = 8;
 constexpr int FAR_BIN0 = AG_NEINT;          // bins below this belong to the near kernel
 constexpr float FAR_T0 = (float)AG_NEINT;   // t = A_DIV * r threshold, same meaning
 constexpr float TINY_T2 = 1.0e-20f;         // keeps rsqrt finite for coincident points
-constexpr float FAR_MAX_T = (float)(AG_NDIEL - 1);
 // The guarded far kernel clamps t half a bin past the last table bin, so that
 // both guard bins of a clamped pair are the last bin (the reference clamps
 // the bin, min(lookup(r), NDIEL-1), main.cpp:2956).

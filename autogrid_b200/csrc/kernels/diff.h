@@ -79,7 +79,6 @@ struct DiffArgs {
     int slot_map[DF_MAXS];       // output map index
     int slot_kind[DF_MAXS];      // DK_*
     int slot_tab[DF_MAXS];       // atom-map index of the pair term (-1: none)
-    int slot_mm[DF_MAXS];        // min/max register or -1
     int slot_desolv[DF_MAXS];    // 1: receives a desolvation term
     double slot_sp[DF_MAXS], slot_vp[DF_MAXS];
     uint8_t act[DF_MAXS][16];    // [slot][hbond + 8 * disorder]

@@ -4,11 +4,11 @@
 // (The FP32 kernels are in diff_rows.cu.)
 //   k_closest_h         closest DS/D1 atom of each point, FP64, the reference's
 //                       scan (main.cpp:2986-3015: file order, strict <)
-//   k_near_lin<R>       forward: a brick of 8x8x4 points per block, one point per
+//   k_near_lin          forward: a brick of 8x8x4 points per block, one point per
 //                       thread; candidate atoms of the cells within 8.05 A of the
 //                       brick staged through shared memory; records for each
 //                       H-bond min/max slot the atoms attaining the min and max
-//   k_near_lin_adj<R>   adjoint: same bricks and staging, pair terms recomputed;
+//   k_near_lin_adj      adjoint: same bricks and staging, pair terms recomputed;
 //                       per candidate the 32 points of a warp are reduced with
 //                       shuffles and one lane adds the atom's gradient (FP64
 //                       atomics); the Hramp gradient on the closest hydrogen's
@@ -25,26 +25,25 @@ using namespace dfm;
 
 namespace {
 
-template <class R> struct NearLinSmem {
-    Atom<R> at[DF_STAGE];
+struct NearLinSmem {
+    Atom<double> at[DF_STAGE];
     BrickSegs sg;
     unsigned short wl[DF_WARPS][DF_STAGE];  // per warp: staged slots near its points
-    R wbox[DF_WARPS][6];                    // per warp: its points' box (lo xyz, hi xyz), A
+    double wbox[DF_WARPS][6];               // per warp: its points' box (lo xyz, hi xyz), A
 };
 
 // This warp's points as a box (lanes outside the grid do not count), kept in
 // shared memory for warp_candidates.
-template <class R>
-__device__ __forceinline__ void warp_box(const Brick &bk, R px, R py, R pz, NearLinSmem<R> &sm)
+__device__ __forceinline__ void warp_box(const Brick &bk, double px, double py, double pz, NearLinSmem &sm)
 {
-    const R big = (R)3.0e38f;
-    R lo[3] = {bk.valid ? px : big, bk.valid ? py : big, bk.valid ? pz : big};
-    R hi[3] = {bk.valid ? px : -big, bk.valid ? py : -big, bk.valid ? pz : -big};
+    const double big = 3.0e38f;
+    double lo[3] = {bk.valid ? px : big, bk.valid ? py : big, bk.valid ? pz : big};
+    double hi[3] = {bk.valid ? px : -big, bk.valid ? py : -big, bk.valid ? pz : -big};
 #pragma unroll
     for (int d = 0; d < 3; d++)
 #pragma unroll
         for (int o = 16; o; o >>= 1) {
-            const R a = __shfl_xor_sync(0xffffffffu, lo[d], o), b = __shfl_xor_sync(0xffffffffu, hi[d], o);
+            const double a = __shfl_xor_sync(0xffffffffu, lo[d], o), b = __shfl_xor_sync(0xffffffffu, hi[d], o);
             lo[d] = a < lo[d] ? a : lo[d];
             hi[d] = b > hi[d] ? b : hi[d];
         }
@@ -61,25 +60,24 @@ __device__ __forceinline__ void warp_box(const Brick &bk, R px, R py, R pz, Near
 // of this warp's box, in staged order (called by all 32 lanes).  Every pair a
 // lane of the warp evaluates (r^2 <= 64 in geom) is on the list, so the pairs
 // and their order are those of the whole chunk.
-template <class R>
-__device__ __forceinline__ int warp_candidates(NearLinSmem<R> &sm, int n)
+__device__ __forceinline__ int warp_candidates(NearLinSmem &sm, int n)
 {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const R *bx = sm.wbox[w];
-    const R lim2 = (R)((AG_NBC + 0.01) * (AG_NBC + 0.01));
+    const double *bx = sm.wbox[w];
+    const double lim2 = (AG_NBC + 0.01) * (AG_NBC + 0.01);
     int cnt = 0;
     for (int j0 = 0; j0 < n; j0 += 32) {
         const int j = j0 + lane;
         bool keep = false;
         if (j < n) {
-            const Atom<R> &at = sm.at[j];
-            R e[3];
-            const R c[3] = {at.x, at.y, at.z};
+            const Atom<double> &at = sm.at[j];
+            double e[3];
+            const double c[3] = {at.x, at.y, at.z};
 #pragma unroll
             for (int d = 0; d < 3; d++) {
-                const R u = bx[d] - c[d], v = c[d] - bx[3 + d];
-                const R m = u > v ? u : v;
-                e[d] = m > (R)0 ? m : (R)0;
+                const double u = bx[d] - c[d], v = c[d] - bx[3 + d];
+                const double m = u > v ? u : v;
+                e[d] = m > 0.0 ? m : 0.0;
             }
             keep = e[0] * e[0] + e[1] * e[1] + e[2] * e[2] <= lim2;
         }
@@ -92,18 +90,17 @@ __device__ __forceinline__ int warp_candidates(NearLinSmem<R> &sm, int n)
 }
 
 // Stage candidates [c0, c0 + DF_STAGE) of the brick into shared memory.
-template <class R>
-__device__ void stage_chunk(const DiffArgs &a, const ConfView &v, NearLinSmem<R> &sm, int c0)
+__device__ void stage_chunk(const DiffArgs &a, const ConfView &v, NearLinSmem &sm, int c0)
 {
     const int k = c0 + threadIdx.x;
     if (threadIdx.x < DF_STAGE && k < sm.sg.total) {
         const int ia = brick_atom(v, sm.sg, k);
-        Atom<R> &t = sm.at[threadIdx.x];
-        t.x = (R)v.x[ia]; t.y = (R)v.y[ia]; t.z = (R)v.z[ia];
-        t.q = (R)v.q[ia]; t.vol = (R)a.vol[ia]; t.solpar = (R)a.solpar[ia];
+        Atom<double> &t = sm.at[threadIdx.x];
+        t.x = v.x[ia]; t.y = v.y[ia]; t.z = v.z[ia];
+        t.q = v.q[ia]; t.vol = a.vol[ia]; t.solpar = a.solpar[ia];
         for (int i = 0; i < 3; i++) {
-            t.rv[i] = (R)v.rv[3 * ia + i];
-            t.rv2[i] = (R)v.rv2[3 * ia + i];
+            t.rv[i] = v.rv[3 * ia + i];
+            t.rv2[i] = v.rv2[3 * ia + i];
         }
         t.meta = a.meta[ia];
         t.idx = ia;
@@ -111,30 +108,29 @@ __device__ void stage_chunk(const DiffArgs &a, const ConfView &v, NearLinSmem<R>
 }
 
 // MS slots and MM min/max registers per point.
-template <class R, int MS, int MM, int MINB>
+template <int MS, int MM, int MINB>
 __global__ void __launch_bounds__(DF_THREADS, MINB)
-k_near_lin(DiffArgs a, const R2<R> *__restrict__ vdw, const R2<R> *__restrict__ sol, R *__restrict__ maps,
+k_near_lin(DiffArgs a, const R2<double> *__restrict__ vdw, const R2<double> *__restrict__ sol, double *__restrict__ maps,
            const int *__restrict__ chs, int *__restrict__ mmarg)
 {
     constexpr int MMA = MM > 0 ? MM : 1;
-    __shared__ NearLinSmem<R> sm;
+    __shared__ NearLinSmem sm;
     const Brick bk = brick_of(a);
     const ConfView v = conf_view(a, DiffGrads{}, bk.conf);
     chs += bk.conf * a.P;
     maps += (long long)bk.conf * a.n_maps_out * a.P;
     mmarg += 2LL * bk.conf * a.n_mm * a.P;
-    const R px = (R)((bk.ix - a.nex) * a.spacing), py = (R)((bk.iy - a.ney) * a.spacing),
-            pz = (R)((bk.iz - a.nez) * a.spacing);
+    const double px = (bk.ix - a.nex) * a.spacing, py = (bk.iy - a.ney) * a.spacing, pz = (bk.iz - a.nez) * a.spacing;
     const int ch = bk.valid ? chs[bk.lin] : -1;
-    R rvh[3] = {0, 0, 0};
+    double rvh[3] = {0, 0, 0};
     if (ch >= 0)
-        for (int i = 0; i < 3; i++) rvh[i] = (R)v.rv[3 * ch + i];
-    R E[MS], hmin[MMA], hmax[MMA];
+        for (int i = 0; i < 3; i++) rvh[i] = v.rv[3 * ch + i];
+    double E[MS], hmin[MMA], hmax[MMA];
     int amin[MMA], amax[MMA];
 #pragma unroll
     for (int s = 0; s < MS; s++) E[s] = 0;
 #pragma unroll
-    for (int s = 0; s < MMA; s++) { hmin[s] = (R)999999.; hmax[s] = (R)-999999.; amin[s] = -1; amax[s] = -1; }
+    for (int s = 0; s < MMA; s++) { hmin[s] = 999999.; hmax[s] = -999999.; amin[s] = -1; amax[s] = -1; }
 
     brick_segments(a, v, bk, sm.sg);
     warp_box(bk, px, py, pz, sm);
@@ -147,63 +143,62 @@ k_near_lin(DiffArgs a, const R2<R> *__restrict__ vdw, const R2<R> *__restrict__ 
         if (!bk.valid) continue;
         const unsigned short *wl = sm.wl[threadIdx.x >> 5];
         for (int k = 0; k < cnt; k++) {
-            const Atom<R> at = sm.at[wl[k]];
-            Geom<R> g;
+            const Atom<double> at = sm.at[wl[k]];
+            Geom<double> g;
             if (!geom(a.need_sol ? sol : nullptr, at, px, py, pz, g)) continue;
-            Ang<R> an;
+            Ang<double> an;
             angular((at.meta >> DM_HB_SHIFT) & 7, (at.meta >> DM_REXP_SHIFT) & 7, (at.meta & DM_DIS) != 0,
                     ch >= 0 && at.idx != ch, g.dn, at.rv, at.rv2, rvh, an);
-            pair_fwd<R, MS, MM>(a, vdw, g, at, an, E, hmin, hmax, amin, amax);
+            pair_fwd<double, MS, MM>(a, vdw, g, at, an, E, hmin, hmax, amin, amax);
         }
     }
     if (!bk.valid) return;
 #pragma unroll
     for (int s = 0; s < MS; s++) {
         if (s >= a.n_slots) break;
-        R v = E[s];
+        double v = E[s];
         if (s < MM && s < a.n_mm) {
             // H-bond finaliser, main.cpp:3420-3431
-            if (amin[s] >= 0) v += hmin[s] + (hmax[s] > (R)0 ? hmax[s] : (R)0);
+            if (amin[s] >= 0) v += hmin[s] + (hmax[s] > 0.0 ? hmax[s] : 0.0);
             mmarg[(2LL * s) * a.P + bk.lin] = amin[s];
-            mmarg[(2LL * s + 1) * a.P + bk.lin] = hmax[s] > (R)0 ? amax[s] : -1;
+            mmarg[(2LL * s + 1) * a.P + bk.lin] = hmax[s] > 0.0 ? amax[s] : -1;
         }
-        if (a.slot_kind[s] == DK_COV) v += covalent_value<R>(a, px, py, pz);
+        if (a.slot_kind[s] == DK_COV) v += covalent_value<double>(a, px, py, pz);
         maps[(long long)a.slot_map[s] * a.P + bk.lin] = v;
     }
 }
 
-template <class R> __device__ __forceinline__ R warp_sum(R v)
+__device__ __forceinline__ double warp_sum(double v)
 {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
 
-template <class R, int MS, int MM, int MINB>
+template <int MS, int MM, int MINB>
 __global__ void __launch_bounds__(DF_THREADS, MINB)
-k_near_lin_adj(DiffArgs a, const R2<R> *__restrict__ vdw, const R2<R> *__restrict__ sol,
-               const R *__restrict__ g_maps, const int *__restrict__ chs, const int *__restrict__ mmarg,
+k_near_lin_adj(DiffArgs a, const R2<double> *__restrict__ vdw, const R2<double> *__restrict__ sol,
+               const double *__restrict__ g_maps, const int *__restrict__ chs, const int *__restrict__ mmarg,
                DiffGrads gr_all)
 {
     constexpr int MMA = MM > 0 ? MM : 1;
-    __shared__ NearLinSmem<R> sm;
+    __shared__ NearLinSmem sm;
     const Brick bk = brick_of(a);
     const ConfView v = conf_view(a, gr_all, bk.conf);
     const DiffGrads gr = v.g;
     chs += bk.conf * a.P;
     g_maps += (long long)bk.conf * a.n_maps_out * a.P;
     mmarg += 2LL * bk.conf * a.n_mm * a.P;
-    const R px = (R)((bk.ix - a.nex) * a.spacing), py = (R)((bk.iy - a.ney) * a.spacing),
-            pz = (R)((bk.iz - a.nez) * a.spacing);
+    const double px = (bk.ix - a.nex) * a.spacing, py = (bk.iy - a.ney) * a.spacing, pz = (bk.iz - a.nez) * a.spacing;
     const int ch = bk.valid ? chs[bk.lin] : -1;
-    R rvh[3] = {0, 0, 0}, g_rvh[3] = {0, 0, 0};
+    double rvh[3] = {0, 0, 0}, g_rvh[3] = {0, 0, 0};
     if (ch >= 0)
-        for (int i = 0; i < 3; i++) rvh[i] = (R)v.rv[3 * ch + i];
-    R gs[MS];
+        for (int i = 0; i < 3; i++) rvh[i] = v.rv[3 * ch + i];
+    double gs[MS];
     int amin[MMA], amax[MMA];
 #pragma unroll
     for (int s = 0; s < MS; s++)
-        gs[s] = (bk.valid && s < a.n_slots) ? g_maps[(long long)a.slot_map[s] * a.P + bk.lin] : (R)0;
+        gs[s] = (bk.valid && s < a.n_slots) ? g_maps[(long long)a.slot_map[s] * a.P + bk.lin] : 0.0;
 #pragma unroll
     for (int s = 0; s < MMA; s++) {
         const bool has = bk.valid && s < MM && s < a.n_mm;
@@ -222,27 +217,27 @@ k_near_lin_adj(DiffArgs a, const R2<R> *__restrict__ vdw, const R2<R> *__restric
         const int cnt = warp_candidates(sm, n);
         const unsigned short *wl = sm.wl[threadIdx.x >> 5];
         for (int k = 0; k < cnt; k++) {
-            const Atom<R> at = sm.at[wl[k]];
-            Geom<R> g;
+            const Atom<double> at = sm.at[wl[k]];
+            Geom<double> g;
             const bool in = bk.valid && geom(a.need_sol ? sol : nullptr, at, px, py, pz, g);
             if (!__any_sync(0xffffffffu, in)) continue;
             const int hb = (at.meta >> DM_HB_SHIFT) & 7;
             const bool dis = (at.meta & DM_DIS) != 0;
-            R g_d[3] = {0, 0, 0}, g_rv[3] = {0, 0, 0}, g_rv2[3] = {0, 0, 0}, G_q = 0;
+            double g_d[3] = {0, 0, 0}, g_rv[3] = {0, 0, 0}, g_rv2[3] = {0, 0, 0}, G_q = 0;
             if (in) {
-                Ang<R> an;
+                Ang<double> an;
                 angular(hb, (at.meta >> DM_REXP_SHIFT) & 7, dis, ch >= 0 && at.idx != ch, g.dn, at.rv, at.rv2, rvh, an);
-                R G_x = 0, G_racc = 0, G_rdon = 0, G_H = 0;
-                pair_bwd<R, MS, MM>(a, vdw, g, at, an, gs, amin, amax, G_x, G_racc, G_rdon, G_H, G_q);
-                R g_dn[3] = {0, 0, 0};
+                double G_x = 0, G_racc = 0, G_rdon = 0, G_H = 0;
+                pair_bwd<double, MS, MM>(a, vdw, g, at, an, gs, amin, amax, G_x, G_racc, G_rdon, G_H, G_q);
+                double g_dn[3] = {0, 0, 0};
                 angular_bwd(hb, dis, an, G_racc, G_rdon, G_H, g.dn, at.rv, at.rv2, rvh, g_dn, g_rv, g_rv2, g_rvh);
                 geom_bwd(g, G_x, g_dn, g_d);
             }
             // the candidate is the same for the whole warp: reduce, one lane adds
             // G_q comes from desolvation terms only
-            const R sx = warp_sum(g_d[0]), sy = warp_sum(g_d[1]), sz = warp_sum(g_d[2]);
-            const R sq = a.need_sol ? warp_sum(G_q) : (R)0;
-            R sr[3] = {0, 0, 0}, sr2[3] = {0, 0, 0};
+            const double sx = warp_sum(g_d[0]), sy = warp_sum(g_d[1]), sz = warp_sum(g_d[2]);
+            const double sq = a.need_sol ? warp_sum(G_q) : 0.0;
+            double sr[3] = {0, 0, 0}, sr2[3] = {0, 0, 0};
             const bool has_rv = hb == 2 || hb == 4 || hb == 5;
             const bool has_rv2 = hb == 5 && !dis;
             if (has_rv)
@@ -251,19 +246,19 @@ k_near_lin_adj(DiffArgs a, const R2<R> *__restrict__ vdw, const R2<R> *__restric
                 for (int i = 0; i < 3; i++) sr2[i] = warp_sum(g_rv2[i]);
             if (lane == 0) {
                 const long long ia = at.idx;
-                atomicAdd(gr.xyz + 3 * ia, (double)sx);
-                atomicAdd(gr.xyz + 3 * ia + 1, (double)sy);
-                atomicAdd(gr.xyz + 3 * ia + 2, (double)sz);
-                if (sq != (R)0) atomicAdd(gr.q + ia, (double)sq);
+                atomicAdd(gr.xyz + 3 * ia, sx);
+                atomicAdd(gr.xyz + 3 * ia + 1, sy);
+                atomicAdd(gr.xyz + 3 * ia + 2, sz);
+                if (sq != 0.0) atomicAdd(gr.q + ia, sq);
                 if (has_rv)
-                    for (int i = 0; i < 3; i++) atomicAdd(gr.rv + 3 * ia + i, (double)sr[i]);
+                    for (int i = 0; i < 3; i++) atomicAdd(gr.rv + 3 * ia + i, sr[i]);
                 if (has_rv2)
-                    for (int i = 0; i < 3; i++) atomicAdd(gr.rv2 + 3 * ia + i, (double)sr2[i]);
+                    for (int i = 0; i < 3; i++) atomicAdd(gr.rv2 + 3 * ia + i, sr2[i]);
             }
         }
     }
-    if (ch >= 0 && (g_rvh[0] != (R)0 || g_rvh[1] != (R)0 || g_rvh[2] != (R)0))
-        for (int i = 0; i < 3; i++) atomicAdd(gr.rv + 3LL * ch + i, (double)g_rvh[i]);
+    if (ch >= 0 && (g_rvh[0] != 0.0 || g_rvh[1] != 0.0 || g_rvh[2] != 0.0))
+        for (int i = 0; i < 3; i++) atomicAdd(gr.rv + 3LL * ch + i, g_rvh[i]);
 }
 
 constexpr int CH_THREADS = 256;
@@ -330,7 +325,7 @@ cudaError_t launch_near_lin(const DiffArgs &a, const void *vdw, const void *sol,
                             cudaStream_t s)
 {
     if (a.P == 0 || a.n_slots == 0) return cudaSuccess;
-    const auto kernel = near_lin_small(a) ? k_near_lin<double, 8, 4, 2> : k_near_lin<double, DF_MAXS, DF_MAXMM, 1>;
+    const auto kernel = near_lin_small(a) ? k_near_lin<8, 4, 2> : k_near_lin<DF_MAXS, DF_MAXMM, 1>;
     kernel<<<brick_grid(a), DF_THREADS, 0, s>>>(a, (const R2<double> *)vdw, (const R2<double> *)sol, maps, ch, mmarg);
     return cudaGetLastError();
 }
@@ -339,7 +334,7 @@ cudaError_t launch_near_lin_adj(const DiffArgs &a, const void *vdw, const void *
                                 const int *mmarg, DiffGrads g, cudaStream_t s)
 {
     if (a.P == 0 || a.n_slots == 0) return cudaSuccess;
-    const auto kernel = near_lin_small(a) ? k_near_lin_adj<double, 8, 4, 2> : k_near_lin_adj<double, DF_MAXS, DF_MAXMM, 1>;
+    const auto kernel = near_lin_small(a) ? k_near_lin_adj<8, 4, 2> : k_near_lin_adj<DF_MAXS, DF_MAXMM, 1>;
     kernel<<<brick_grid(a), DF_THREADS, 0, s>>>(a, (const R2<double> *)vdw, (const R2<double> *)sol, g_maps, ch, mmarg, g);
     return cudaGetLastError();
 }

@@ -1,7 +1,9 @@
 // Per-pair arithmetic of the differentiable mode (kernels/diff.h states the
 // mode): directional factors of main.cpp:3075-3272 with their partial
 // derivatives, and the chain rule from the factors back to the pair vector and
-// the bond vectors.  Written once for FP32 and FP64, host and device.
+// the bond vectors, written once for FP32 and FP64, host and device; and the
+// geometry and table terms of a pair in FP64 (the FP32 kernels have their own,
+// diff_rows.cu).
 #pragma once
 #include <cmath>
 
@@ -251,26 +253,12 @@ template <class R> struct Geom {
 };
 
 // r = max(|d|, DF_TINY) and 1 / r from r^2.  r is the correctly rounded
-// square root everywhere (it picks the table bin, and the adjoint's slopes
-// jump at bin edges); FP32 on the device takes 1 / r from one rsqrt.approx
-// (about 2 ulp) instead of a division.
+// square root (it picks the table bin, and the adjoint's slopes jump at bin edges).
 DF_HD void dist_inv(double r2, double &r, double &inv)
 {
     r = sqrt(r2);
     if (r < DF_TINY) r = DF_TINY;
     inv = 1.0 / r;
-}
-DF_HD void dist_inv(float r2, float &r, float &inv)
-{
-#ifdef __CUDA_ARCH__
-    r = sqrtf(r2);
-    if (r < float(DF_TINY)) r = float(DF_TINY);
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(r * r));
-#else
-    r = sqrtf(r2);
-    if (r < float(DF_TINY)) r = float(DF_TINY);
-    inv = 1.0f / r;
-#endif
 }
 
 // False when the pair adds nothing: beyond 8 A, or a disordered hydrogen that

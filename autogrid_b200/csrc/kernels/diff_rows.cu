@@ -34,6 +34,7 @@
 #include "diff_pair.cuh"
 
 #include "diff_brick.cuh"
+#include "table_row.cuh"
 #include "type_sort.cuh"
 #include "warp_sums.cuh"
 
@@ -42,21 +43,6 @@ namespace agb {
 using namespace dfm;
 
 namespace {
-
-struct alignas(32) Row8 {
-    float2 p[4];
-};
-
-// 8 consecutive floats of a 32-byte aligned table row.
-__device__ __forceinline__ Row8 load_row8(const float *p)
-{
-    Row8 r;
-    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-        : "=f"(r.p[0].x), "=f"(r.p[0].y), "=f"(r.p[1].x), "=f"(r.p[1].y), "=f"(r.p[2].x), "=f"(r.p[2].y),
-          "=f"(r.p[3].x), "=f"(r.p[3].y)
-        : "l"(p));
-    return r;
-}
 
 __device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
 
