@@ -2,8 +2,10 @@
 //
 // Frames.  The grid is tiled into frames of FRAME_X x FRAME_Y x FRAME_Z points.
 // Inside a frame, atom and grid-point coordinates are expressed relative to
-// the frame's first point, in units of distance-table bins (1/A_DIV Angstrom),
-// and rounded to FP32 by one canonical routine.  The far-field e-map kernel
+// one of its points, in units of distance-table bins (1/A_DIV Angstrom), and
+// rounded to FP32 by one canonical routine.  That point is the frame's middle,
+// FRAME_X/2 and so on, in the far and near kernels, its first point in the
+// differentiable e map.  The far-field e-map kernel
 // and the near-field (short-range) kernel both decide "is this pair far?"
 // from exactly the same FP32 operations on exactly the same FP32 inputs, so
 // every (point, atom) pair is counted by exactly one of them.

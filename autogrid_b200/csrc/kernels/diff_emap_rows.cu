@@ -281,17 +281,17 @@ k_elin_adj(DiffArgs a, const float2 *__restrict__ gtab, cudaTextureObject_t tex,
             const int nb = min(32, na - ib);
 #pragma unroll 1
             for (int ii = 0; ii < nb; ii++) {
-                    const float4 A = s_atom[ib + ii];
-                    const float2 dy = __fadd2_rn(both(A.x), P.npy);
-                    const float dz = A.y + P.npz;
-                    const float2 s = __ffma2_rn(dy, dy, both(__fmaf_rn(dz, dz, TINY_T2)));
-                    const bool close = __any_sync(0xffffffffu, fminf(s.x, s.y) < 4096.f);
-                    // in bins, with inv = min(1/r, 1/64): sum of w inv T, and of
-                    // k = w inv / r (T' - T / r) (without T / r where r < 64), k dx
-                    float2 aq = both(0.f), ax = both(0.f), k0 = both(0.f), k1 = both(0.f);
-                    auto pairs = [&](auto near) {
-                constexpr bool CLOSE = decltype(near)::value;
-                auto add = [&](int r, float2 h, float2 rs, float2 T, float2 d, float2 dx) {
+                const float4 A = s_atom[ib + ii];
+                const float2 dy = __fadd2_rn(both(A.x), P.npy);
+                const float dz = A.y + P.npz;
+                const float2 s = __ffma2_rn(dy, dy, both(__fmaf_rn(dz, dz, TINY_T2)));
+                const bool close = __any_sync(0xffffffffu, fminf(s.x, s.y) < 4096.f);
+                // in bins, with inv = min(1/r, 1/64): sum of w inv T, and of
+                // k = w inv / r (T' - T / r) (without T / r where r < 64), k dx
+                float2 aq = both(0.f), ax = both(0.f), k0 = both(0.f), k1 = both(0.f);
+                auto pairs = [&](auto near) {
+                    constexpr bool CLOSE = decltype(near)::value;
+                    auto add = [&](int r, float2 h, float2 rs, float2 T, float2 d, float2 dx) {
                         float2 out = rs;
                         if (CLOSE) out = make_float2(rs.x < 0.015625f ? rs.x : 0.f, rs.y < 0.015625f ? rs.y : 0.f);
                         aq = __ffma2_rn(h, T, aq);
@@ -309,7 +309,7 @@ k_elin_adj(DiffArgs a, const float2 *__restrict__ gtab, cudaTextureObject_t tex,
                         for (int r = 0; r < 2; r++) {
                             const int n = 2 * j + r;
                             float2 t2 = __ffma2_rn(dx, dx, both(r ? s.y : s.x));
-                        if (CLOSE) t2 = make_float2(fmaxf(t2.x, ER_MIN_T2), fmaxf(t2.y, ER_MIN_T2));
+                            if (CLOSE) t2 = make_float2(fmaxf(t2.x, ER_MIN_T2), fmaxf(t2.y, ER_MIN_T2));
                             const float2 rs = make_float2(rsqrt_approx(t2.x), rsqrt_approx(t2.y));
                             float2 f, inv = rs;
                             uint32_t b0, b1;
@@ -341,7 +341,7 @@ k_elin_adj(DiffArgs a, const float2 *__restrict__ gtab, cudaTextureObject_t tex,
                 if (close) pairs(std::true_type{});
                 else pairs(std::false_type{});
                 const float s0 = k0.x + k0.y, s1 = k1.x + k1.y;
-                    float sum[4] = {ax.x + ax.y, fmaf(dy.x, s0, dy.y * s1), dz * (s0 + s1), aq.x + aq.y};
+                float sum[4] = {ax.x + ax.y, fmaf(dy.x, s0, dy.y * s1), dz * (s0 + s1), aq.x + aq.y};
                 const float total = warp_sums(sum, lane);
                 if ((lane & 7) == 0) {
                     const int n = lane >> 3, at = t0 + ib + ii;

@@ -25,11 +25,11 @@
 // What bounds it: the forward, the L1 data path of the row gathers (85% busy, at
 // one wavefront per lane for a 32-byte gather that hits L1, two for a miss);
 // the adjoint, issue (64%) and that path (69%).  Eight conformers of 8,000
-// atoms, 101^3 points, 8 Vina maps: forward 3.1 ms, adjoint 3.0 ms; kernels that
+// atoms, 101^3 points, 8 Vina maps: forward 2.8 ms, adjoint 2.8 ms; kernels that
 // walked the slots of every pair one by one took 8.6 and 12.8 ms (295 and 475
 // instructions per warp and candidate, now 65 and 101).  Rows in the order of
 // the candidates' cells instead of their types, and step rows in the forward,
-// hit L1 for 58% instead of 89%: forward 3.6 ms.  4,000 atoms, 61^3 points,
+// hit L1 for 58% instead of 89%: the forward took 3.6 ms in place of 3.1.  4,000 atoms, 61^3 points,
 // 8 AD4 maps: 0.39 -> 0.17 ms and 0.75 -> 0.33 ms.
 #include "diff_pair.cuh"
 

@@ -22,7 +22,7 @@
 //                (deterministic; lets the far and near kernels run
 //                concurrently).
 // k_emap_exact -- FP64 twin: every pair with the reference's bin, double table,
-//                file order summation.
+//                summed in file order within an atom chunk, chunks in order.
 #include <algorithm>
 
 #include "agb_device.cuh"
@@ -73,9 +73,9 @@ __device__ __forceinline__ int far_exact_bin(const double *ax128, const double *
     return (int)__dmul_rn(r, (double)AG_A_DIV) | FAR_TIE_FLAG;
 }
 
-// A thread's place in a far-field unit: the compact 4x4x2 lane footprint per
-// warp (fewest table bank conflicts); each thread holds 8 points of one
-// x-row, x = tx + 8j and tx + 8j + 4 (j < EF_PAIRS).
+// A thread's place in the fix-up: the compact 4x4x2 lane footprint per warp;
+// each thread stands for 8 points of one x-row, x = tx + 8j and tx + 8j + 4
+// (j < EF_PAIRS), one of the two rows that a thread of the far kernel holds.
 struct FarLane {
     int tx, ty, tz;
     bool warp_in;  // some row and plane of the warp lie inside the box
@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(EF_THREADS, EF_MIN_CTAS) k_emap_far(FarArgs a)
 
 // ------------------------------------------------------------- fix-up ---
 // The far pairs the guard flagged, resolved after the far-field kernel.  One
-// CTA per far-field unit (frame, chunk), with the far kernel's lane layout.
+// CTA per far-field unit (frame, chunk), a thread for each row of 8 points (far_lane).
 // Each warp collects its threads' flagged (thread, atom) items from the edge
 // bits into a shared list and processes them 32 at a time, one per lane:
 // first the owner thread's pairs with that atom are re-evaluated by the far

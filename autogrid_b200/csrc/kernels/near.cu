@@ -25,10 +25,10 @@ struct NearSmem {
 // One 8x8x4 brick of points, one thread per point:
 //   stage  candidate atoms of the cells within 8.05 A of the brick, with
 //          frame-relative FP32 coordinates for the filters
-//   A      closest DS/D1 atom per point (main.cpp:2986-3015): any DS/D1 atom
-//          within 8.05 A of the point is a candidate, so a best distance
+//   A      closest DS/D1 atom per point (main.cpp:2986-3015) among the candidates:
+//          any DS/D1 atom within 8.05 A of the point is one, so a best distance
 //          <= 8 A is the global minimum; strict '<' in file order == lowest
-//          index on a tie; other points scan all DS/D1 atoms
+//          index on a tie.  Where no DS/D1 atom is a candidate, no pair asks for it
 //   B      pair terms of every candidate inside 8 A
 // Only classes with an H-bond action evaluate the directional factors.
 __global__ void __launch_bounds__(NB_THREADS, 2) k_near_exact(DevProblem p_, NearGroup g, NearPtrs ptr)

@@ -80,7 +80,7 @@ static __device__ __noinline__ void angular_exact(const DevProblem &p, int ia, i
             if (e == 2) o.racc = __dmul_rn(cos_theta, cos_theta);
             else if (e == 4) { const double t = __dmul_rn(cos_theta, cos_theta); o.racc = __dmul_rn(t, t); }
             else o.racc = cos_theta;
-            if (ia == ch || ch < 0) {  // ch < 0 only when no ligand map needs Hramp
+            if (ia == ch || ch < 0) {  // ch < 0: no DS/D1 candidate in reach, then no pair comes here
                 o.Hramp = 1.;
             } else {
                 const double *rh = p.rv + 3 * (size_t)ch;

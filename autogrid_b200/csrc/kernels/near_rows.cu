@@ -42,7 +42,10 @@ constexpr int NR_THREADS = 256;
 // nothing spills and L1 keeps 156 KB for the table rows; 3 (80 registers)
 // take 2.40 against 1.94 ms (127^3 points, 10,000 atoms, 16 maps), 4 2.87 ms.
 constexpr int NEAR_MIN_CTAS = 2;
-constexpr int NR_CHUNK = 320;           // candidates staged at once (most bricks need one chunk)
+// Candidates staged at once.  Most bricks need one chunk at 0.026 atoms per A^3;
+// at 0.06, the inside of a protein with its hydrogens, most need two (10,000
+// atoms, 127^3 points, 16 maps, serial: 1.75 ms at 0.026, 2.78 at 0.042, 3.76 at 0.06).
+constexpr int NR_CHUNK = 320;
 constexpr int NR_WARPS = NR_THREADS / 32;
 constexpr int NR_SEGS = NB_SEGS_MAX;    // cell rows laid out at once
 constexpr float GUARD_COS = 5.0e-5f;
@@ -719,8 +722,8 @@ k_near_batch(const NearInst *__restrict__ insts, const long long *__restrict__ u
 }
 
 // Accumulators a launch holds per point: groups of at most 8 maps (the
-// 8-map sets of batched ensembles) run with 8, which frees 8 of the 80
-// registers; larger groups with NG_MAX.
+// 8-map sets of batched ensembles) run with 8, one row load per pair instead of
+// two; larger groups with NG_MAX.
 constexpr int NGK_SMALL = 8;
 
 template <int BX, int BY, int BZ>
